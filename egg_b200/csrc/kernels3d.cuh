@@ -13,6 +13,7 @@
 // blend (src/sweep.hpp:1534-1650).
 #pragma once
 
+#include "dof3.cuh"
 #include "entity3.cuh"
 #include "kernels2d.cuh"
 #include "metric3.cuh"
@@ -72,65 +73,45 @@ __device__ __forceinline__ void edges3(const Tile3Shared<TI, TJ, TK>& sm, int bu
     }
 }
 
-// fp32 edge matrix of sample b from the window's fp32 forward edges
-// fe[(3k + i) * N + node] = (X[node + e_k] - X[node])_i.  Column k of T is
-// the forward edge along k at the corner with bit k cleared, so this is
-// bitwise the fp32 rounding of edges3's fp64 column: the cache saves each
-// sample 12 fp64 loads, 9 subtractions and 9 conversions.
-template <int TI, int TJ, int TK>
-__device__ __forceinline__ void edges3f(const float* __restrict__ fe, int bu, int bv, int bw, int b, float t[9])
+// Whether a corner sample of the cell with base window node n is inverted or
+// badly shaped: det T <= 0 or det^2 < kBadCell^2 times its columns' squared
+// lengths, from the window's fp32 forward edges fe[(3 k + i) N + node] =
+// (X[node + e_k] - X[node])_i.  Sample b's columns are the cell's edges along
+// axis k at the corner b without bit k, so the cell's 12 edges and their
+// lengths are formed once, and the two samples along axis 2 share one
+// instruction (a sample at a time from 9 loads each took 11% of the kernel).
+template <class W> __device__ __forceinline__ bool cell_bad3(const float* __restrict__ fe, int n)
 {
-    using W = Win3<TI, TJ, TK>;
+    using L = Lane<F2>;
+    const EdgeF<W::N> E {fe};
+    F2 e0[2][3], n0[2];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const int c = b & ~bit3(k);
-        const int id = W::idx(bu + (c >> 2), bv + ((c >> 1) & 1), bw + (c & 1));
-#pragma unroll
-        for (int i = 0; i < 3; ++i) { t[3 * i + k] = fe[(3 * k + i) * W::N + id]; }
+    for (int b = 0; b < 2; ++b) {
+        E.get(0, n + b * W::WK, n + b * W::WK + 1, e0[b]);
+        n0[b] = dotv(e0[b], e0[b]);
     }
-}
-
-template <class R> __device__ __forceinline__ bool below3(const R t[9], R det, R thr)
-{
-    R n[3];
+    bool bad = false;
 #pragma unroll
-    for (int k = 0; k < 3; ++k) { n[k] = t[k] * t[k] + t[3 + k] * t[3 + k] + t[6 + k] * t[6 + k]; }
-    return !(det > R(0)) || det * det < thr * thr * n[0] * n[1] * n[2];
-}
-
-// Bit b set: sample b of the cell with base (bu, bv, bw) is inverted or
-// badly shaped (below3 at kBadCell), from the fp32 edge cache; the det is
-// formed as shared3 forms it (first cofactor row).
-template <int TI, int TJ, int TK>
-__device__ __forceinline__ unsigned cell_bad3(const float* __restrict__ fe, int bu, int bv, int bw)
-{
-    unsigned mask = 0u;
+    for (int a = 0; a < 2; ++a) {
+        const int m = n + a * W::WJ * W::WK;
+        F2 e1[3], m1[3];
+        E.get(3 * W::N, m, m + 1, e1);
+        negv(e1, m1);
+        const F2 n1 = dotv(e1, e1);
 #pragma unroll
-    for (int b = 0; b < 8; ++b) {
-        float t[9];
-        edges3f<TI, TJ, TK>(fe, bu, bv, bw, b, t);
-        const float c0 = t[4] * t[8] - t[5] * t[7];
-        const float c1 = t[5] * t[6] - t[3] * t[8];
-        const float c2 = t[3] * t[7] - t[4] * t[6];
-        const float D = t[0] * c0 + t[1] * c1 + t[2] * c2;
-        if (below3<float>(t, D, float(kBadCell))) { mask |= 1u << b; }
+        for (int b = 0; b < 2; ++b) {
+            F2 e2[3], c[3];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) { e2[i] = L::set(fe[(6 + i) * W::N + m + b * W::WK]); }
+            crossv(m1, e1, e0[b], c);  // e0 x e1
+            const F2 D = dotv(e2, c), nn = n0[b] * n1 * dotv(e2, e2);
+            const F2 t = vfma(D, D, L::set(-float(kBadCell * kBadCell)) * nn);
+            bad = bad || !(D.v.x > 0.0f) || !(D.v.y > 0.0f) || t.v.x < 0.0f || t.v.y < 0.0f;
+        }
     }
-    return mask;
+    return bad;
 }
 
-template <int KIND, class R>
-__device__ __forceinline__ void sample3_shared(const double t64[9], double delta, Shared3<R>& S)
-{
-    R t[9];
-#pragma unroll
-    for (int i = 0; i < 9; ++i) { t[i] = R(t64[i]); }
-    shared3<R>(KIND, t, R(delta), S);
-}
-
-// Complete update of one interior DOF at window node (1+ti, 1+tj, 1+tk) in
-// working precision R.  Returns false (and leaves `out` untouched) when R is
-// float and the patch holds an inverted or badly shaped sample, so the caller
-// redoes the DOF in fp64.
 // fp64 metric change of one near-degenerate trial sample (cell base
 // (bu, bv, bw), corner b, the DOF at corner a moved from pos by d), from the
 // staged fp64 positions.  Out of line: it runs rarely and its fp64
@@ -150,236 +131,178 @@ __device__ __noinline__ float dmu3_guard64(const Tile3Shared<TI, TJ, TK>& sm, in
     return float(m1 - m0);
 }
 
-template <int TI, int TJ, int TK, int KIND, class R>
-__device__ bool dof3_update(const Tile3Shared<TI, TJ, TK>& sm, const float* __restrict__ fe,
-                            const uint8_t* __restrict__ cbad, int ti, int tj, int tk, const double tau[3],
-                            double delta, double omega, double out[3], bool grad_only = false)
+// Whether one corner sample admits a move of the DOFs that do not move it:
+// its metric is finite and, outside the untangle phase, its det positive.
+template <int KIND> __device__ __forceinline__ bool sample_ok64(const double t[9], double delta)
+{
+    const double c0 = t[4] * t[8] - t[5] * t[7], c1 = t[5] * t[6] - t[3] * t[8], c2 = t[3] * t[7] - t[4] * t[6];
+    const double D = t[0] * c0 + t[1] * c1 + t[2] * c2;
+    if constexpr (KIND != kUntangle) {
+        if (!(D > 0.0)) { return false; }
+        double s = 0.0;
+#pragma unroll
+        for (int k = 0; k < 9; ++k) { s += t[k] * t[k]; }
+        // q <= s^2 / 3, so the metric cannot overflow here
+        if (s < 1e100 && D * D > 1e-280 * (s * s * s)) { return true; }
+    }
+    double d;
+    return isfinite(mu3_value<double>(KIND, t, delta, d));
+}
+
+// Bit b set: sample b of the window cell with base (bu, bv, bw) fails
+// sample_ok64.
+template <int TI, int TJ, int TK, int KIND>
+__device__ __forceinline__ unsigned cell_stop64(const Tile3Shared<TI, TJ, TK>& sm, int bu, int bv, int bw, double delta)
+{
+    const double none[3] = {0.0, 0.0, 0.0};
+    unsigned mask = 0u;
+#pragma unroll 2
+    for (int b = 0; b < 8; ++b) {
+        double t[9];
+        edges3<TI, TJ, TK>(sm, bu, bv, bw, b, -1, none, t);
+        if (!sample_ok64<KIND>(t, delta)) { mask |= 1u << b; }
+    }
+    return mask;
+}
+
+// The samples of a cell that do not move its corner a, as bits of cell_stop64.
+__device__ __forceinline__ constexpr unsigned still_bits(int a)
+{
+    return (1u << (a ^ 7)) | (1u << (a ^ 6)) | (1u << (a ^ 5)) | (1u << (a ^ 3));
+}
+
+// fp64 update (or, grad_only, gradient) of the DOF at window node p.
+// `stop`: a sample around it that it does not move rules
+// every step out.  The accept test compares the energies of the 32 samples it
+// moves; the other 32 add the same constant to both sides.
+template <int TI, int TJ, int TK, int KIND>
+__device__ __forceinline__ void dof3_fp64(const Tile3Shared<TI, TJ, TK>& sm, int p, bool stop, const double tau[3],
+                                          double delta, double omega, double out[3], bool grad_only)
 {
     using W = Win3<TI, TJ, TK>;
-    const int pid = W::idx(ti + 1, tj + 1, tk + 1);
-    const double pos[3] = {sm.P[0][pid], sm.P[1][pid], sm.P[2][pid]};
-    R g[3] = {R(0), R(0), R(0)};
-    R h[6] = {R(0), R(0), R(0), R(0), R(0), R(0)};
-    R e0 = R(0), econst = R(0);
-    R mdconst = R(INFINITY);
-    const double none[3] = {0.0, 0.0, 0.0};
-    if constexpr (std::is_same_v<R, float>) {
-        // Every sample of the DOF's 8 cells is in its patch (4 move it, 4 do
-        // not).  If any is inverted or badly shaped the DOF relaxes in fp64;
-        // otherwise the samples that do not move it have positive dets and
-        // the fp32 accept test needs nothing else from them (it sums metric
-        // changes, and their min det cannot decide the sign of the trial min).
-        unsigned bad = 0u;
+    const EdgeD<W::N> E {&sm.P[0][0]};
+    double g[3], h[6], e0;
+    if (grad_only) {
+        dof3_system<W, KIND, true>(E, p, delta, g, h, e0);
 #pragma unroll
-        for (int cell = 0; cell < 8; ++cell) {
-            bad |= cbad[W::cidx(ti + (cell >> 2), tj + ((cell >> 1) & 1), tk + (cell & 1))];
-        }
-        if (bad) { return false; }
-    } else {
-    // Samples that do not move the DOF: constant energy and det.
-#pragma unroll 1
-    for (int cell = 0; cell < 8; ++cell) {
-        const int ci = cell >> 2, cj = (cell >> 1) & 1, ck = cell & 1;
-        const int a = ((1 - ci) << 2) | ((1 - cj) << 1) | (1 - ck);
-#pragma unroll
-        for (int x = 0; x < 4; ++x) {
-            const int b = a ^ (x == 0 ? 7 : (x == 1 ? 6 : (x == 2 ? 5 : 3)));
-            Shared3<R> S;
-            if constexpr (std::is_same_v<R, float>) {
-                float tf[9];
-                edges3f<TI, TJ, TK>(fe, ti + ci, tj + cj, tk + ck, b, tf);
-                shared3<float>(KIND, tf, float(delta), S);
-            } else {
-                double t[9];
-                edges3<TI, TJ, TK>(sm, ti + ci, tj + cj, tk + ck, b, -1, none, t);
-                sample3_shared<KIND, R>(t, delta, S);
-            }
-            econst += mu3_from<R>(KIND, S);
-            mdconst = fmin(mdconst, S.D);
-        }
+        for (int q = 0; q < 3; ++q) { out[q] = g[q] - tau[q]; }
+        return;
     }
-    }
-    // Samples that move it: role r (0 corner, 1+k axis-k neighbour).
+    dof3_system<W, KIND, false>(E, p, delta, g, h, e0);
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-#pragma unroll 1
-        for (int cell = 0; cell < 8; ++cell) {
-            const int ci = cell >> 2, cj = (cell >> 1) & 1, ck = cell & 1;
-            const int a = ((1 - ci) << 2) | ((1 - cj) << 1) | (1 - ck);
-            const int b = r == 0 ? a : (a ^ bit3(r - 1));
-            Shared3<R> S;
-            if constexpr (std::is_same_v<R, float>) {
-                float tf[9];
-                edges3f<TI, TJ, TK>(fe, ti + ci, tj + cj, tk + ck, b, tf);
-                shared3<float>(KIND, tf, float(delta), S);
-            } else {
-                double t[9];
-                edges3<TI, TJ, TK>(sm, ti + ci, tj + cj, tk + ck, b, -1, none, t);
-                sample3_shared<KIND, R>(t, delta, S);
-            }
-            e0 += mu3_from<R>(KIND, S);
-            R v[3];
+    for (int q = 0; q < 3; ++q) { g[q] -= tau[q]; }
 #pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                const R sk = (b & bit3(k)) ? R(-1) : R(1);
-                v[k] = r == 0 ? -sk : (k == r - 1 ? sk : R(0));
-            }
-            R gg[3], hh[6];
-            role3<R>(KIND, S, v, gg, hh, r - 1);  // r >= 1: v = sk e_(r-1)
-#pragma unroll
-            for (int q = 0; q < 3; ++q) { g[q] += gg[q]; }
-#pragma unroll
-            for (int q = 0; q < 6; ++q) { h[q] += hh[q]; }
-        }
-    }
-    e0 += econst;
-    const R gv[3] = {g[0] - R(tau[0]), g[1] - R(tau[1]), g[2] - R(tau[2])};
-    if (grad_only) {  // gradient-only mode (FAS restriction / tau)
-        out[0] = double(gv[0]);
-        out[1] = double(gv[1]);
-        out[2] = double(gv[2]);
-        return true;
-    }
-    R dl[3];
-    solve3<R>(h, gv, dl);
-    R alpha = R(1);
-    if constexpr (std::is_same_v<R, float>) {
-        // fp32: accept on the summed metric changes of the 32 samples the DOF
-        // moves, with the fp64 energy tolerance.  The move is rank one along
-        // the line, so each sample reduces to a few coefficients
-        // (line_sample3) and every step length costs a few flops; two step
-        // lengths (alpha, alpha / 2) are tried per pass, in the reference's
-        // order.  Near-degenerate trial samples are differenced in fp64.
-        const float u[3] = {dl[0], dl[1], dl[2]};
-        // pass 0 tries alpha = 1 alone (almost every DOF accepts it); later
-        // passes try two step lengths each, 10 in all in the reference's order
-        int tried = 0;
-#pragma unroll 1
-        for (int pass = 0; tried < 10; ++pass) {
-            const int nt = (pass == 0 || tried == 9) ? 1 : 2;
-            const float al[2] = {alpha, 0.5f * alpha};
-            float dsum0 = 0.0f, dsum1 = 0.0f;
-            float md0 = mdconst, md1 = mdconst;
-            unsigned long long guard = 0ull;  // bit 2 * sample + trial
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-#pragma unroll 1
-                for (int cell = 0; cell < 8; ++cell) {
-                    const int ci = cell >> 2, cj = (cell >> 1) & 1, ck = cell & 1;
-                    const int a = ((1 - ci) << 2) | ((1 - cj) << 1) | (1 - ck);
-                    const int b = r == 0 ? a : (a ^ bit3(r - 1));
-                    float tt[9], v[3];
-                    edges3f<TI, TJ, TK>(fe, ti + ci, tj + cj, tk + ck, b, tt);
-#pragma unroll
-                    for (int k = 0; k < 3; ++k) {
-                        const float sk = (b & bit3(k)) ? -1.0f : 1.0f;
-                        v[k] = r == 0 ? -sk : (k == r - 1 ? sk : 0.0f);
-                    }
-                    LineSample3<float> L;
-                    line_sample3<float>(tt, u, v, L, r - 1);
-#pragma unroll
-                    for (int tr = 0; tr < 2; ++tr) {
-                        if (tr >= nt) { break; }
-                        float dn;
-                        const float dm = dmu3_at<float>(KIND, L, al[tr], float(delta), dn);
-                        float nrm[3];
-                        line_norms3<float>(L, al[tr], nrm, r - 1);
-                        if (!(fabsf(dn) > 0.0f) ||
-                            dn * dn < float(kGuard * kGuard) * nrm[0] * nrm[1] * nrm[2]) {
-                            guard |= 1ull << (2 * (r * 8 + cell) + tr);
-                        } else if (tr == 0) {
-                            dsum0 += dm;
-                            md0 = fminf(md0, dn);
-                        } else {
-                            dsum1 += dm;
-                            md1 = fminf(md1, dn);
-                        }
-                    }
-                }
-            }
-#pragma unroll 1
-            for (int bit = 0; guard != 0ull && bit < 64; ++bit) {
-                if (!((guard >> bit) & 1ull)) { continue; }
-                const int si = bit >> 1, tr = bit & 1;
-                const int r = si >> 3, cell = si & 7;
-                const int ci = cell >> 2, cj = (cell >> 1) & 1, ck = cell & 1;
-                const int a = ((1 - ci) << 2) | ((1 - cj) << 1) | (1 - ck);
-                const int b = r == 0 ? a : (a ^ bit3(r - 1));
-                const double d3[3] = {double(al[tr] * u[0]), double(al[tr] * u[1]), double(al[tr] * u[2])};
-                float dn;
-                const float dm = dmu3_guard64<TI, TJ, TK, KIND>(sm, ti + ci, tj + cj, tk + ck, b, a, pos, d3, delta, dn);
-                if (tr == 0) {
-                    dsum0 += dm;
-                    md0 = fminf(md0, dn);
-                } else {
-                    dsum1 += dm;
-                    md1 = fminf(md1, dn);
-                }
-            }
-#pragma unroll
-            for (int tr = 0; tr < 2; ++tr) {
-                if (tr >= nt) { break; }
-                const float d3[3] = {al[tr] * u[0], al[tr] * u[1], al[tr] * u[2]};
-                const float ds = tr == 0 ? dsum0 : dsum1, mdt = tr == 0 ? md0 : md1;
-                const float dd = ds - (float(tau[0]) * d3[0] + float(tau[1]) * d3[1] + float(tau[2]) * d3[2]);
-                if (isfinite(dd) && dd <= float(Tol<double>::energy) && (KIND == kUntangle || mdt > 0.0f)) {
-                    out[0] = pos[0] + omega * double(d3[0]);
-                    out[1] = pos[1] + omega * double(d3[1]);
-                    out[2] = pos[2] + omega * double(d3[2]);
-                    return true;
-                }
-            }
-            tried += nt;
-            alpha *= nt == 1 ? 0.5f : 0.25f;
-        }
-    } else {
+    for (int q = 0; q < 3; ++q) { out[q] = sm.P[q][p]; }
+    if (stop) { return; }
+    double dl[3];
+    solve3<double>(h, g, dl);
+    double alpha = 1.0;
 #pragma unroll 1
     for (int it = 0; it < 10; ++it) {
-        const double d[3] = {double(alpha * dl[0]), double(alpha * dl[1]), double(alpha * dl[2])};
-        const double trial[3] = {pos[0] + d[0], pos[1] + d[1], pos[2] + d[2]};
-        R e = econst;
-        R md = mdconst;
+        const double d[3] = {alpha * dl[0], alpha * dl[1], alpha * dl[2]};
+        double md = INFINITY;
+        const double e =
+          dof3_trial<W, KIND>(E, p, d, delta, md) - (tau[0] * d[0] + tau[1] * d[1] + tau[2] * d[2]);
+        if (isfinite(e) && e <= e0 + Tol<double>::energy && (KIND == kUntangle || md > 0.0)) {
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
+            for (int q = 0; q < 3; ++q) { out[q] += omega * d[q]; }
+            return;
+        }
+        alpha *= 0.5;
+    }
+}
+
+// The mixed path's DOFs next to an inverted or badly shaped sample: fp64, out
+// of line so that its registers do not weigh on the fp32 path.
+template <int TI, int TJ, int TK, int KIND>
+__device__ __noinline__ void dof3_fallback64(const Tile3Shared<TI, TJ, TK>& sm, int ti, int tj, int tk,
+                                             const double tau[3], double delta, double omega, double out[3],
+                                             bool grad_only)
+{
+    bool stop = false;
 #pragma unroll 1
-            for (int cell = 0; cell < 8; ++cell) {
-                const int ci = cell >> 2, cj = (cell >> 1) & 1, ck = cell & 1;
-                const int a = ((1 - ci) << 2) | ((1 - cj) << 1) | (1 - ck);
-                const int b = r == 0 ? a : (a ^ bit3(r - 1));
-                double t[9];
-                edges3<TI, TJ, TK>(sm, ti + ci, tj + cj, tk + ck, b, a, trial, t);
-                R tt[9];
+    for (int cell = 0; cell < 8 && !grad_only; ++cell) {
+        stop = stop || (cell_stop64<TI, TJ, TK, KIND>(sm, ti + (cell >> 2), tj + ((cell >> 1) & 1), tk + (cell & 1),
+                                                      delta) &
+                        still_bits(7 - cell)) != 0u;
+    }
+    dof3_fp64<TI, TJ, TK, KIND>(sm, Win3<TI, TJ, TK>::idx(ti + 1, tj + 1, tk + 1), stop, tau, delta, omega, out,
+                                grad_only);
+}
+
+// The line search's pass over near-degenerate trial samples, out of line: the
+// fp32 sum without them plus their changes differenced in fp64.
+template <int TI, int TJ, int TK, int KIND>
+__device__ __noinline__ float dof3_line_guard(const Tile3Shared<TI, TJ, TK>& sm, const float* __restrict__ fe, int ti,
+                                              int tj, int tk, const float d[3], double delta, float& md)
+{
+    using W = Win3<TI, TJ, TK>;
+    const EdgeF<W::N> E {fe};
+    const int p = W::idx(ti + 1, tj + 1, tk + 1);
+    float low = 0.0f, add = 0.0f;
+    unsigned guard = 0u;
+    md = INFINITY;
+    const float ds = dof3_line<W, KIND, true>(E, p, d, float(delta), md, low, guard);
+    const double pos[3] = {sm.P[0][p], sm.P[1][p], sm.P[2][p]};
+    const double d3[3] = {double(d[0]), double(d[1]), double(d[2])};
+    while (guard != 0u) {
+        const int bit = __ffs(int(guard)) - 1;
+        guard &= guard - 1u;
+        const int cell = bit & 7, r = bit >> 3, a = 7 - cell, b = r == 0 ? a : (a ^ bit3(r - 1));
+        float dn;
+        add += dmu3_guard64<TI, TJ, TK, KIND>(sm, ti + (cell >> 2), tj + ((cell >> 1) & 1), tk + (cell & 1), b, a,
+                                              pos, d3, delta, dn);
+        md = fminf(md, dn);
+    }
+    return ds + add;
+}
+
+// fp32 update (or gradient) of a DOF whose 8 cells hold no bad sample: the
+// samples that it does not move then have positive dets, and the accept test
+// sums metric changes, with the fp64 energy tolerance.  Near-degenerate trial
+// samples are differenced in fp64.
+template <int TI, int TJ, int TK, int KIND>
+__device__ __forceinline__ void dof3_fp32(const Tile3Shared<TI, TJ, TK>& sm, const float* __restrict__ fe, int ti,
+                                          int tj, int tk, const double tau[3], double delta, double omega,
+                                          double out[3], bool grad_only)
+{
+    using W = Win3<TI, TJ, TK>;
+    const EdgeF<W::N> E {fe};
+    const int p = W::idx(ti + 1, tj + 1, tk + 1);
+    const float fd = float(delta);
+    float g[3], h[6];
+    const float ft[3] = {float(tau[0]), float(tau[1]), float(tau[2])};
+    if (grad_only) {
+        dof3_system<W, KIND, true>(E, p, fd, g, h);
 #pragma unroll
-                for (int q = 0; q < 9; ++q) { tt[q] = R(t[q]); }
-                R det;
-                R m = mu3_value<R>(KIND, tt, R(delta), det);
-                if constexpr (std::is_same_v<R, float>) {
-                    // fp64 re-evaluation of near-degenerate trial samples: the
-                    // barrier decision needs the sign of det exactly.
-                    if (!(fabsf(det) > 0.0f) || below3<float>(tt, fabsf(det), float(kGuard))) {
-                        double d64;
-                        m = float(mu3_value<double>(KIND, t, delta, d64));
-                        det = d64 > 0.0 ? fmaxf(float(d64), 1e-38f) : (d64 < 0.0 ? fminf(float(d64), -1e-38f) : 0.0f);
-                    }
-                }
-                e += m;
-                md = fmin(md, det);
-            }
-        }
-        e -= R(tau[0]) * R(d[0]) + R(tau[1]) * R(d[1]) + R(tau[2]) * R(d[2]);
-        if (isfinite(e) && e <= e0 + Tol<R>::energy && (KIND == kUntangle || md > R(0))) {
-            out[0] = pos[0] + omega * d[0];
-            out[1] = pos[1] + omega * d[1];
-            out[2] = pos[2] + omega * d[2];
-            return true;
-        }
-        alpha *= R(0.5);
+        for (int q = 0; q < 3; ++q) { out[q] = double(g[q] - ft[q]); }
+        return;
     }
+    dof3_system<W, KIND, false>(E, p, fd, g, h);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) { g[q] -= ft[q]; }
+    float dl[3];
+    solve3<float>(h, g, dl);
+    float alpha = 1.0f;
+#pragma unroll 1
+    for (int it = 0; it < 10; ++it) {
+        const float d[3] = {alpha * dl[0], alpha * dl[1], alpha * dl[2]};
+        float md = INFINITY, low = INFINITY;
+        unsigned none_guard = 0u;
+        float ds = dof3_line<W, KIND, false>(E, p, d, fd, md, low, none_guard);
+        if (!(low > 0.0f) || !isfinite(ds)) {
+            ds = dof3_line_guard<TI, TJ, TK, KIND>(sm, fe, ti, tj, tk, d, delta, md);
+        }
+        ds -= ft[0] * d[0] + ft[1] * d[1] + ft[2] * d[2];
+        if (isfinite(ds) && ds <= float(Tol<double>::energy) && (KIND == kUntangle || md > 0.0f)) {
+#pragma unroll
+            for (int q = 0; q < 3; ++q) { out[q] = sm.P[q][p] + omega * double(d[q]); }
+            return;
+        }
+        alpha *= 0.5f;
     }
-    out[0] = pos[0];
-    out[1] = pos[1];
-    out[2] = pos[2];
-    return true;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) { out[q] = sm.P[q][p]; }
 }
 
 template <int TI, int TJ, int TK, int MINB, int KIND, class C>
@@ -391,7 +314,7 @@ __global__ void __launch_bounds__(TI* TJ* TK, MINB)
     using W = Win3<TI, TJ, TK>;
     __shared__ Tile3Shared<TI, TJ, TK> sm;
     __shared__ float fe[std::is_same_v<C, float> ? 9 * W::N : 1];  // fp32 forward edges (mixed)
-    __shared__ uint8_t cbad[std::is_same_v<C, float> ? W::NC : 1];  // per window cell: bad-sample bits (mixed)
+    __shared__ uint8_t cbad[W::NC];  // per window cell: bad-sample bits (mixed), stop bits (fp64)
     const Tile3 tile = tiles[blockIdx.x];
     const BlockInfo bi = blocks[tile.block];
     const int n0 = bi.n[0], n1 = bi.n[1], n2 = bi.n[2];
@@ -432,10 +355,15 @@ __global__ void __launch_bounds__(TI* TJ* TK, MINB)
         // past the block hold zero positions and are read by no DOF
         for (int c = threadIdx.x; c < W::NC; c += NT) {
             const int cu = c / ((W::WJ - 1) * (W::WK - 1)), cv = (c / (W::WK - 1)) % (W::WJ - 1), cw = c % (W::WK - 1);
-            cbad[c] = uint8_t(cell_bad3<TI, TJ, TK>(fe, cu, cv, cw));
+            cbad[c] = cell_bad3<W>(fe, W::idx(cu, cv, cw)) ? 1 : 0;
         }
-        __syncthreads();
+    } else {
+        for (int c = threadIdx.x; c < W::NC; c += NT) {
+            const int cu = c / ((W::WJ - 1) * (W::WK - 1)), cv = (c / (W::WK - 1)) % (W::WJ - 1), cw = c % (W::WK - 1);
+            cbad[c] = uint8_t(cell_stop64<TI, TJ, TK, KIND>(sm, cu, cv, cw, delta));
+        }
     }
+    __syncthreads();
     const int ti = threadIdx.x / (TJ * TK), tj = (threadIdx.x / TK) % TJ, tk = threadIdx.x % TK;
     const int gi = tile.i0 + ti, gj = tile.j0 + tj, gk = tile.k0 + tk;
     if (gi > n0 - 2 || gj > n1 - 2 || gk > n2 - 2) { return; }
@@ -449,8 +377,18 @@ __global__ void __launch_bounds__(TI* TJ* TK, MINB)
     }
     double out[3];
     const bool go = grad_out != nullptr;
-    if (!dof3_update<TI, TJ, TK, KIND, C>(sm, fe, cbad, ti, tj, tk, tv, delta, omega, out, go)) {
-        dof3_update<TI, TJ, TK, KIND, double>(sm, nullptr, nullptr, ti, tj, tk, tv, delta, omega, out, go);
+    unsigned bad = 0u;
+#pragma unroll
+    for (int cell = 0; cell < 8; ++cell) {
+        const unsigned m = cbad[W::cidx(ti + (cell >> 2), tj + ((cell >> 1) & 1), tk + (cell & 1))];
+        bad |= std::is_same_v<C, float> ? m : m & still_bits(7 - cell);
+    }
+    if constexpr (std::is_same_v<C, double>) {
+        dof3_fp64<TI, TJ, TK, KIND>(sm, W::idx(ti + 1, tj + 1, tk + 1), bad != 0u, tv, delta, omega, out, go);
+    } else if (bad != 0u) {
+        dof3_fallback64<TI, TJ, TK, KIND>(sm, ti, tj, tk, tv, delta, omega, out, go);
+    } else {
+        dof3_fp32<TI, TJ, TK, KIND>(sm, fe, ti, tj, tk, tv, delta, omega, out, go);
     }
     double* dst = go ? grad_out : Xout;
     dst[3 * slot] = out[0];

@@ -112,8 +112,12 @@ constexpr int kNumVariants = EGG_B200_NUM_VARIANTS;
 constexpr int kMaxCopyThreads = 16;
 constexpr Variant kVar64[kNumVariants] = {{8, 16, 1, 5, 1}, {8, 16, 1, 4}, {8, 16, 1, 5}, {8, 16, 1, 6}, {8, 16, 1, 4, 1}};
 constexpr Variant kVar32[kNumVariants] = {{8, 16, 1, 7, 2}, {8, 16, 1, 8, 2}, {8, 16, 1, 6, 2}, {8, 16, 1, 5, 2}, {8, 16, 1, 7, 3}};
-constexpr Variant kVar3_64[kNumVariants] = {{4, 8, 8, 1}, {4, 8, 8, 2}, {2, 8, 16, 2}, {2, 8, 16, 3}, {2, 4, 16, 4}};
-constexpr Variant kVar3_32[kNumVariants] = {{4, 8, 8, 1}, {4, 8, 8, 2}, {2, 8, 16, 2}, {2, 8, 16, 3}, {2, 4, 16, 4}};
+// 3D (interior3_kernel), us a sweep of a 129^3 / 59^3 / 33^3 cube, in the table's
+// order: fp64 969 / 125 / 25.0, 957 / 112 / 26.9, 963 / 120 / 27.0,
+// 1029 / 120 / 28.3, 975 / 125 / 27.2; mixed 545 / 72 / 16.8, 556 / 72 / 16.7,
+// 559 / 74 / 16.7, 558 / 69 / 17.1, 582 / 73 / 17.0.
+constexpr Variant kVar3_64[kNumVariants] = {{4, 8, 8, 2}, {2, 4, 16, 4}, {4, 4, 8, 4}, {2, 4, 8, 8}, {2, 8, 16, 2}};
+constexpr Variant kVar3_32[kNumVariants] = {{4, 4, 8, 4}, {2, 4, 16, 4}, {4, 8, 8, 2}, {4, 4, 4, 8}, {2, 8, 16, 2}};
 
 enum KernelId {
     kKInterior = 0,
