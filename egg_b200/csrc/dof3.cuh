@@ -357,7 +357,7 @@ struct AxisTurn {
 };
 template <class W> __device__ __forceinline__ AxisTurn axis_turn()
 {
-    return AxisTurn {W::WJ * W::WK, W::WK, 1, 0, 3 * W::N, 6 * W::N, 4, 2, 1};
+    return AxisTurn {W::S0, W::S1, W::S2, 0, 3 * W::N, 6 * W::N, 4, 2, 1};
 }
 
 // Newton system of the DOF at window node p: gradient g[3] and Hessian h[6]
@@ -376,7 +376,7 @@ __device__ __forceinline__ void dof3_system(const EdgeF<W::N>& E, int p, float d
 #pragma unroll 1
         for (int c = 0; c < 4; ++c) {
             const float s0 = (c & 2) ? 1.0f : -1.0f, s1 = (c & 1) ? 1.0f : -1.0f;
-            const int na = (c & 2) ? p : p - W::WJ * W::WK, nb = (c & 1) ? p : p - W::WK;
+            const int na = (c & 2) ? p : p - W::S0, nb = (c & 1) ? p : p - W::S1;
             F2 o0[3], o1[3];
 #pragma unroll
             for (int m = 0; m < 3; ++m) {
@@ -411,25 +411,40 @@ __device__ __forceinline__ void dof3_system(const EdgeF<W::N>& E, int p, float d
 }
 
 // fp64; e: the energy of the 32 moving samples without their constant -1.
-template <class W, int KIND, bool GRAD>
-__device__ __forceinline__ void dof3_system(const EdgeD<W::N>& E, int p, double delta, double g[3], double h[6],
-                                            double& e)
+// NH = 2: two neighbouring threads share the DOF, each with one side of every
+// group and one direction of axis 2 at the corner (`half`); both end with the
+// same totals and take the same decisions.
+__device__ __forceinline__ unsigned pair_mask() { return 3u << (threadIdx.x & 30u); }
+template <int NH> __device__ __forceinline__ double pair_sum(double v)
+{
+    if constexpr (NH == 2) { v += __shfl_xor_sync(pair_mask(), v, 1, 2); }
+    return v;
+}
+template <int NH> __device__ __forceinline__ double pair_min(double v)
+{
+    if constexpr (NH == 2) { v = fmin(v, __shfl_xor_sync(pair_mask(), v, 1, 2)); }
+    return v;
+}
+
+template <class W, int KIND, int NH, bool GRAD>
+__device__ __forceinline__ void dof3_system(const EdgeD<W::N>& E, int p, int half, double delta, double g[3],
+                                            double h[6], double& e)
 {
     Sys3<double> S;
     S.clear();
 #pragma unroll 1
-    for (int c = 0; c < 8; ++c) {
+    for (int c = 4 * half; c < 4 * half + 8 / NH; ++c) {
         double o0[3], o1[3], o2[3];
-        E.get(p, (c & 2) ? p + W::WJ * W::WK : p - W::WJ * W::WK, o0);
-        E.get(p, (c & 1) ? p + W::WK : p - W::WK, o1);
-        E.get(p, (c & 4) ? p + 1 : p - 1, o2);
+        E.get(p, (c & 2) ? p + W::S0 : p - W::S0, o0);
+        E.get(p, (c & 1) ? p + W::S1 : p - W::S1, o1);
+        E.get(p, (c & 4) ? p + W::S2 : p - W::S2, o2);
         const double sig = (__popc(c) & 1) ? 1.0 : -1.0;  // product of the three edge signs
         corner_system<KIND, GRAD>(o0, o1, o2, sig, delta, S);
     }
     AxisTurn t = axis_turn<W>();
 #pragma unroll 1
-    for (int k = 0; k < 6; ++k) {
-        const bool up = (k & 1) != 0;
+    for (int k = 0; k < 6 / NH; ++k) {
+        const bool up = NH == 2 ? half != 0 : (k & 1) != 0;
         const int n = up ? p + t.sk : p - t.sk;
         double tk[3], ti[2][3], tj[2][3];
         E.get(up ? p : n, up ? n : p, tk);
@@ -438,16 +453,18 @@ __device__ __forceinline__ void dof3_system(const EdgeD<W::N>& E, int p, double 
         E.get(n - t.sj, n, tj[0]);
         E.get(n, n + t.sj, tj[1]);
         axis_system<KIND, GRAD>(tk, ti, tj, up ? -1.0 : 1.0, delta, S);
-        if (up) { t.next(); }
+        if (NH == 2 || up) { t.next(); }
     }
     constexpr double n9 = 1.0 / 9.0;
 #pragma unroll
-    for (int m = 0; m < 3; ++m) { g[m] = n9 * S.g[m]; }
+    for (int m = 0; m < 3; ++m) { g[m] = n9 * pair_sum<NH>(S.g[m]); }
+    if constexpr (!GRAD) {
 #pragma unroll
-    for (int m = 0; m < 6; ++m) {
-        h[m] = n9 * ((m == 0 || m == 3 || m == 5) ? 2.0 * (S.A[m] + S.hI) : S.A[m]);
+        for (int m = 0; m < 6; ++m) {
+            h[m] = n9 * pair_sum<NH>((m == 0 || m == 3 || m == 5) ? 2.0 * (S.A[m] + S.hI) : S.A[m]);
+        }
+        e = n9 * pair_sum<NH>(S.e);
     }
-    e = n9 * S.e;
 }
 
 // ---------------------------------------------------------------------------
@@ -529,7 +546,7 @@ __device__ __forceinline__ float dof3_line(const EdgeF<W::N>& E, int p, const fl
 #pragma unroll 1
         for (int c = 0; c < 4; ++c) {
             const float s0 = (c & 2) ? 1.0f : -1.0f, s1 = (c & 1) ? 1.0f : -1.0f;
-            const int na = (c & 2) ? p : p - W::WJ * W::WK, nb = (c & 1) ? p : p - W::WK;
+            const int na = (c & 2) ? p : p - W::S0, nb = (c & 1) ? p : p - W::S1;
             F2 o0[3], o1[3], m0[3], m1[3], C0[3], C1[3], C2[3], cs[3];
 #pragma unroll
             for (int m = 0; m < 3; ++m) {
@@ -611,9 +628,9 @@ __device__ __forceinline__ float dof3_line(const EdgeF<W::N>& E, int p, const fl
 }
 
 // fp64: the energy of the 32 moving samples (without their constant -1) with
-// the DOF moved by d, and their smallest det.
-template <class W, int KIND>
-__device__ __forceinline__ double dof3_trial(const EdgeD<W::N>& E, int p, const double d[3], double delta,
+// the DOF moved by d (summed over its NH threads), and this thread's smallest det.
+template <class W, int KIND, int NH>
+__device__ __forceinline__ double dof3_trial(const EdgeD<W::N>& E, int p, int half, const double d[3], double delta,
                                              double& md)
 {
     auto value = [&](double s, double q, double D) {
@@ -627,11 +644,11 @@ __device__ __forceinline__ double dof3_trial(const EdgeD<W::N>& E, int p, const 
     };
     double e = 0.0;
 #pragma unroll 1
-    for (int c = 0; c < 8; ++c) {
+    for (int c = 4 * half; c < 4 * half + 8 / NH; ++c) {
         double o0[3], o1[3], o2[3], m0[3], m1[3], C0[3], C1[3], C2[3];
-        E.get(p, (c & 2) ? p + W::WJ * W::WK : p - W::WJ * W::WK, o0);
-        E.get(p, (c & 1) ? p + W::WK : p - W::WK, o1);
-        E.get(p, (c & 4) ? p + 1 : p - 1, o2);
+        E.get(p, (c & 2) ? p + W::S0 : p - W::S0, o0);
+        E.get(p, (c & 1) ? p + W::S1 : p - W::S1, o1);
+        E.get(p, (c & 4) ? p + W::S2 : p - W::S2, o2);
 #pragma unroll
         for (int m = 0; m < 3; ++m) {
             o0[m] -= d[m];
@@ -648,8 +665,8 @@ __device__ __forceinline__ double dof3_trial(const EdgeD<W::N>& E, int p, const 
     }
     AxisTurn t = axis_turn<W>();
 #pragma unroll 1
-    for (int k = 0; k < 6; ++k) {
-        const bool up = (k & 1) != 0;
+    for (int k = 0; k < 6 / NH; ++k) {
+        const bool up = NH == 2 ? half != 0 : (k & 1) != 0;
         const int n = up ? p + t.sk : p - t.sk;
         double tk[3], tj[2][3], nj[2], yj[2];
         E.get(up ? p : n, up ? n : p, tk);
@@ -677,9 +694,9 @@ __device__ __forceinline__ double dof3_trial(const EdgeD<W::N>& E, int p, const 
                 e += value(nk + N, dotv(c, c) + (N * nk - (yi + yj[b])), dotv(tk, c));
             }
         }
-        if (up) { t.next(); }
+        if (NH == 2 || up) { t.next(); }
     }
-    return e;
+    return pair_sum<NH>(e);
 }
 
 }  // namespace egg_b200

@@ -32,6 +32,7 @@ __host__ __device__ constexpr int bit3(int k) { return 4 >> k; }
 template <int TI, int TJ, int TK> struct Win3 {
     static constexpr int WI = TI + 2, WJ = TJ + 2, WK = TK + 2;
     static constexpr int N = WI * WJ * WK;
+    static constexpr int S0 = WJ * WK, S1 = WK, S2 = 1;  // node strides of the axes
     static constexpr int NC = (WI - 1) * (WJ - 1) * (WK - 1);  // cells of the window
     __device__ static int idx(int u, int v, int w) { return (u * WJ + v) * WK + w; }
     __device__ static int cidx(int u, int v, int w) { return (u * (WJ - 1) + v) * (WK - 1) + w; }
@@ -149,17 +150,22 @@ template <int KIND> __device__ __forceinline__ bool sample_ok64(const double t[9
     return isfinite(mu3_value<double>(KIND, t, delta, d));
 }
 
-// Bit b set: sample b of the window cell with base (bu, bv, bw) fails
+// Bit b set: sample b of the cell with base node n of window P fails
 // sample_ok64.
-template <int TI, int TJ, int TK, int KIND>
-__device__ __forceinline__ unsigned cell_stop64(const Tile3Shared<TI, TJ, TK>& sm, int bu, int bv, int bw, double delta)
+template <class W, int KIND> __device__ __forceinline__ unsigned cell_stop64(const double* P, int n, double delta)
 {
-    const double none[3] = {0.0, 0.0, 0.0};
+    const int st[3] = {W::S0, W::S1, W::S2};
     unsigned mask = 0u;
 #pragma unroll 2
     for (int b = 0; b < 8; ++b) {
+        const int at = n + ((b & 4) ? W::S0 : 0) + ((b & 2) ? W::S1 : 0) + ((b & 1) ? W::S2 : 0);
         double t[9];
-        edges3<TI, TJ, TK>(sm, bu, bv, bw, b, -1, none, t);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const int lo = (b & bit3(k)) ? at - st[k] : at;
+#pragma unroll
+            for (int i = 0; i < 3; ++i) { t[3 * i + k] = P[i * W::N + lo + st[k]] - P[i * W::N + lo]; }
+        }
         if (!sample_ok64<KIND>(t, delta)) { mask |= 1u << b; }
     }
     return mask;
@@ -171,28 +177,27 @@ __device__ __forceinline__ constexpr unsigned still_bits(int a)
     return (1u << (a ^ 7)) | (1u << (a ^ 6)) | (1u << (a ^ 5)) | (1u << (a ^ 3));
 }
 
-// fp64 update (or, grad_only, gradient) of the DOF at window node p.
-// `stop`: a sample around it that it does not move rules
-// every step out.  The accept test compares the energies of the 32 samples it
-// moves; the other 32 add the same constant to both sides.
-template <int TI, int TJ, int TK, int KIND>
-__device__ __forceinline__ void dof3_fp64(const Tile3Shared<TI, TJ, TK>& sm, int p, bool stop, const double tau[3],
+// fp64 update (or, grad_only, gradient) of the DOF at node p of window P, by
+// its NH threads (dof3_system).  `stop`: a sample around it that it does not
+// move rules every step out.  The accept test compares the energies of the 32
+// samples it moves; the other 32 add the same constant to both sides.
+template <class W, int KIND, int NH>
+__device__ __forceinline__ void dof3_fp64(const double* P, int p, int half, bool stop, const double tau[3],
                                           double delta, double omega, double out[3], bool grad_only)
 {
-    using W = Win3<TI, TJ, TK>;
-    const EdgeD<W::N> E {&sm.P[0][0]};
+    const EdgeD<W::N> E {P};
     double g[3], h[6], e0;
     if (grad_only) {
-        dof3_system<W, KIND, true>(E, p, delta, g, h, e0);
+        dof3_system<W, KIND, NH, true>(E, p, half, delta, g, h, e0);
 #pragma unroll
         for (int q = 0; q < 3; ++q) { out[q] = g[q] - tau[q]; }
         return;
     }
-    dof3_system<W, KIND, false>(E, p, delta, g, h, e0);
+    dof3_system<W, KIND, NH, false>(E, p, half, delta, g, h, e0);
 #pragma unroll
     for (int q = 0; q < 3; ++q) { g[q] -= tau[q]; }
 #pragma unroll
-    for (int q = 0; q < 3; ++q) { out[q] = sm.P[q][p]; }
+    for (int q = 0; q < 3; ++q) { out[q] = P[q * W::N + p]; }
     if (stop) { return; }
     double dl[3];
     solve3<double>(h, g, dl);
@@ -202,7 +207,8 @@ __device__ __forceinline__ void dof3_fp64(const Tile3Shared<TI, TJ, TK>& sm, int
         const double d[3] = {alpha * dl[0], alpha * dl[1], alpha * dl[2]};
         double md = INFINITY;
         const double e =
-          dof3_trial<W, KIND>(E, p, d, delta, md) - (tau[0] * d[0] + tau[1] * d[1] + tau[2] * d[2]);
+          dof3_trial<W, KIND, NH>(E, p, half, d, delta, md) - (tau[0] * d[0] + tau[1] * d[1] + tau[2] * d[2]);
+        md = pair_min<NH>(md);
         if (isfinite(e) && e <= e0 + Tol<double>::energy && (KIND == kUntangle || md > 0.0)) {
 #pragma unroll
             for (int q = 0; q < 3; ++q) { out[q] += omega * d[q]; }
@@ -219,15 +225,14 @@ __device__ __noinline__ void dof3_fallback64(const Tile3Shared<TI, TJ, TK>& sm, 
                                              const double tau[3], double delta, double omega, double out[3],
                                              bool grad_only)
 {
+    using W = Win3<TI, TJ, TK>;
     bool stop = false;
 #pragma unroll 1
     for (int cell = 0; cell < 8 && !grad_only; ++cell) {
-        stop = stop || (cell_stop64<TI, TJ, TK, KIND>(sm, ti + (cell >> 2), tj + ((cell >> 1) & 1), tk + (cell & 1),
-                                                      delta) &
-                        still_bits(7 - cell)) != 0u;
+        const int n = W::idx(ti + (cell >> 2), tj + ((cell >> 1) & 1), tk + (cell & 1));
+        stop = stop || (cell_stop64<W, KIND>(&sm.P[0][0], n, delta) & still_bits(7 - cell)) != 0u;
     }
-    dof3_fp64<TI, TJ, TK, KIND>(sm, Win3<TI, TJ, TK>::idx(ti + 1, tj + 1, tk + 1), stop, tau, delta, omega, out,
-                                grad_only);
+    dof3_fp64<W, KIND, 1>(&sm.P[0][0], W::idx(ti + 1, tj + 1, tk + 1), 0, stop, tau, delta, omega, out, grad_only);
 }
 
 // The line search's pass over near-degenerate trial samples, out of line: the
@@ -360,7 +365,7 @@ __global__ void __launch_bounds__(TI* TJ* TK, MINB)
     } else {
         for (int c = threadIdx.x; c < W::NC; c += NT) {
             const int cu = c / ((W::WJ - 1) * (W::WK - 1)), cv = (c / (W::WK - 1)) % (W::WJ - 1), cw = c % (W::WK - 1);
-            cbad[c] = uint8_t(cell_stop64<TI, TJ, TK, KIND>(sm, cu, cv, cw, delta));
+            cbad[c] = uint8_t(cell_stop64<W, KIND>(&sm.P[0][0], W::idx(cu, cv, cw), delta));
         }
     }
     __syncthreads();
@@ -384,7 +389,7 @@ __global__ void __launch_bounds__(TI* TJ* TK, MINB)
         bad |= std::is_same_v<C, float> ? m : m & still_bits(7 - cell);
     }
     if constexpr (std::is_same_v<C, double>) {
-        dof3_fp64<TI, TJ, TK, KIND>(sm, W::idx(ti + 1, tj + 1, tk + 1), bad != 0u, tv, delta, omega, out, go);
+        dof3_fp64<W, KIND, 1>(&sm.P[0][0], W::idx(ti + 1, tj + 1, tk + 1), 0, bad != 0u, tv, delta, omega, out, go);
     } else if (bad != 0u) {
         dof3_fallback64<TI, TJ, TK, KIND>(sm, ti, tj, tk, tv, delta, omega, out, go);
     } else {
@@ -457,14 +462,76 @@ __device__ __forceinline__ void assemble_T3(const double* X, int32_t ic, const i
     }
 }
 
-// Stored-patch sweep, 3D, G lanes per DOF (see stored_patch_kernel): the
-// lanes split the DOF's samples and reduce across the group.
-template <int KIND, int G, bool CON>
-__global__ void stored3_kernel(StoredPatch3 sp, const double* __restrict__ Xin, double* __restrict__ Xout,
-                               const double* __restrict__ tau, double delta, double omega, double* __restrict__ grad_out)
+// Stored DOFs whose patch is a plain 3 x 3 x 3 lattice with identity target
+// and unit weight: nodes off every block edge where two blocks meet (and, on
+// the FAS levels, the same nodes).  Blocks may be turned against one another;
+// the table lists each DOF's 27 node slots in one right-handed order of its
+// own, so the structured update applies (dof3_fp64, two threads per DOF)
+// instead of 64 gathered samples with a general target.
+struct Lattice3 {
+    int64_t n;            // DOFs
+    const int32_t* node;  // [27][n] node slots, entry 13 the DOF
+};
+constexpr int kLatDofs = 64;  // DOFs per CTA of 2 kLatDofs threads
+struct WinLat3 {
+    static constexpr int N = 27 * kLatDofs, S0 = 9 * kLatDofs, S1 = 3 * kLatDofs, S2 = kLatDofs;
+};
+
+template <int KIND>
+__device__ __noinline__ void lattice3_cta(double* P, Lattice3 lat, int64_t d0, const double* __restrict__ Xin,
+                                          double* __restrict__ Xout, const double* __restrict__ tau, double delta,
+                                          double omega, double* __restrict__ grad_out)
 {
+    using W = WinLat3;
+    for (int i = threadIdx.x; i < W::N; i += 2 * kLatDofs) {
+        const int64_t d = d0 + i % kLatDofs;
+        if (d >= lat.n) { continue; }
+        const int64_t s = lat.node[(i / kLatDofs) * lat.n + d];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) { P[q * W::N + i] = Xin[3 * s + q]; }
+    }
+    __syncthreads();
+    const int t = threadIdx.x >> 1, half = threadIdx.x & 1, p = 13 * kLatDofs + t;
+    const int64_t d = d0 + t;
+    if (d >= lat.n) { return; }
+    const int64_t slot = lat.node[13 * lat.n + d];
+    const bool go = grad_out != nullptr;
+    double tv[3] = {0.0, 0.0, 0.0}, out[3];
+    if (tau != nullptr) {
+#pragma unroll
+        for (int q = 0; q < 3; ++q) { tv[q] = tau[3 * slot + q]; }
+    }
+    unsigned stop = 0u;
+#pragma unroll 1
+    for (int c = 0; c < 4 && !go; ++c) {
+        const int cell = 4 * half + c;
+        const int n = p + ((cell & 4) ? 0 : -W::S0) + ((cell & 2) ? 0 : -W::S1) + ((cell & 1) ? 0 : -W::S2);
+        stop |= cell_stop64<W, KIND>(P, n, delta) & still_bits(7 - cell);
+    }
+    stop |= __shfl_xor_sync(pair_mask(), stop, 1, 2);
+    dof3_fp64<W, KIND, 2>(P, p, half, stop != 0u, tv, delta, omega, out, go);
+    if (half) { return; }
+    double* dst = go ? grad_out : Xout;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) { dst[3 * slot + q] = out[q]; }
+}
+
+// Stored-patch sweep, 3D, G lanes per DOF (see stored_patch_kernel): the
+// lanes split the DOF's samples and reduce across the group.  The first `nb`
+// CTAs take the stored DOFs, the others the lattice DOFs.
+template <int KIND, int G, bool CON>
+__global__ void stored3_kernel(StoredPatch3 sp, int nb, Lattice3 lat, const double* __restrict__ Xin,
+                               double* __restrict__ Xout, const double* __restrict__ tau, double delta, double omega,
+                               double* __restrict__ grad_out)
+{
+    if (int(blockIdx.x) >= nb) {
+        extern __shared__ __align__(16) unsigned char lat_smem[];
+        lattice3_cta<KIND>(reinterpret_cast<double*>(lat_smem), lat, int64_t(blockIdx.x - nb) * kLatDofs, Xin, Xout,
+                           tau, delta, omega, grad_out);
+        return;
+    }
     const int lane = threadIdx.x & (G - 1);
-    const int64_t ngroups = (int64_t(gridDim.x) * blockDim.x) / G;
+    const int64_t ngroups = (int64_t(nb) * blockDim.x) / G;
     const double none[3] = {0, 0, 0};
     for (int64_t d = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) / G; d < sp.n; d += ngroups) {
         const int32_t slot = sp.slot[d];

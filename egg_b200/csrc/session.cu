@@ -154,6 +154,10 @@ struct LevelData {
     // interior-kernel variant of a coarse FAS level, tuned on the level's
     // own data (-1: the session's variant)
     int variant = -1;
+    // stored DOFs whose 3D patch is a plain lattice: [27][n_lat] node slots;
+    // not among the n_stored below
+    int64_t n_lat = 0;
+    DevBuf<int32_t> lat_node;
     int64_t n_stored = 0;
     DevBuf<int32_t> st_slot, st_gc, st_gn0, st_gn1, st_gn2, st_role;
     DevBuf<int64_t> st_off;
@@ -586,6 +590,8 @@ static void set_tiles(Session& S, LevelData& L, Variant v)
     L.tile_ck = v.ck;
     L.tile_fd = v.fd;
 }
+
+#include "lattice_host.inc"
 
 static Session* create_session(const egg_b200_session_desc& d)
 {
@@ -1069,6 +1075,14 @@ static Session* create_session(const egg_b200_session_desc& d)
     } else {
         S->st_wtstride = 1;
     }
+    std::vector<int32_t> lat_node;
+    if (D == 3 && !st_slot.empty()) {
+        S->n_lat = split_lattice3(StoredRows3 {st_slot, st_gc, st_gn0, st_gn1, st_gn2, st_role, st_off, st_s0, st_s1,
+                                               st_s2, st_W, st_wt, S->st_wstride != 0, S->st_wtstride != 0, &st_etag,
+                                               &st_epar, soft_terms.empty() ? nullptr : &soft_off},
+                                  lat_node);
+        S->n_stored = int64_t(st_slot.size());
+    }
 
     // ---- energy stencil -------------------------------------------------
     int64_t ncell = 0;
@@ -1294,6 +1308,7 @@ static Session* create_session(const egg_b200_session_desc& d)
     S->free_d.upload(S->free_h);
     S->variant = 0;
     set_tiles(*S, *S, variant_shape(*S, 0));
+    S->lat_node.upload(lat_node);
     S->st_slot.upload(st_slot);
     S->st_off.upload(st_off);
     if (S->n_constrained) {
@@ -1568,7 +1583,7 @@ template <int KIND>
 static void launch_stored(Session& S, LevelData& L, const double* xin, double* xout, const double* tau, double delta,
                           double omega, double* gout = nullptr, cudaStream_t on = nullptr, bool cold = false)
 {
-    if (L.n_stored == 0) { return; }
+    if (L.n_stored + L.n_lat == 0) { return; }
     const cudaStream_t st = on ? on : S.stream;
     const int G = stored_group(L.n_stored, S.dim);
     const unsigned grid = unsigned(std::min<int64_t>((L.n_stored * G + 127) / 128, 148 * 16));
@@ -1579,13 +1594,18 @@ static void launch_stored(Session& S, LevelData& L, const double* xin, double* x
                          L.n_constrained ? L.st_etag.p : nullptr, L.n_constrained ? L.st_epar.p : nullptr,
                          cold ? 1 : 0, soft_view(L), L.n_bspline ? L.arena.p : nullptr,
                          L.n_bspline ? L.seeds.p : nullptr};
+        const Lattice3 lat {L.n_lat, L.lat_node.p};
+        const int nb = L.n_stored ? int(grid) : 0;
+        const unsigned all = unsigned(nb + (L.n_lat + kLatDofs - 1) / kLatDofs);
+        const size_t sm = L.n_lat ? size_t(3 * WinLat3::N) * sizeof(double) : 0;
         auto go3 = [&](auto con) {
             constexpr bool C = decltype(con)::value;
+            static_assert(2 * kLatDofs == 128, "one CTA size for both parts");
             switch (G) {
-            case 32: stored3_kernel<KIND, 32, C><<<grid, 128, 0, st>>>(sp, xin, xout, tau, delta, omega, gout); break;
-            case 8: stored3_kernel<KIND, 8, C><<<grid, 128, 0, st>>>(sp, xin, xout, tau, delta, omega, gout); break;
-            case 2: stored3_kernel<KIND, 2, C><<<grid, 128, 0, st>>>(sp, xin, xout, tau, delta, omega, gout); break;
-            default: stored3_kernel<KIND, 1, C><<<grid, 128, 0, st>>>(sp, xin, xout, tau, delta, omega, gout); break;
+            case 32: stored3_kernel<KIND, 32, C><<<all, 128, sm, st>>>(sp, nb, lat, xin, xout, tau, delta, omega, gout); break;
+            case 8: stored3_kernel<KIND, 8, C><<<all, 128, sm, st>>>(sp, nb, lat, xin, xout, tau, delta, omega, gout); break;
+            case 2: stored3_kernel<KIND, 2, C><<<all, 128, sm, st>>>(sp, nb, lat, xin, xout, tau, delta, omega, gout); break;
+            default: stored3_kernel<KIND, 1, C><<<all, 128, sm, st>>>(sp, nb, lat, xin, xout, tau, delta, omega, gout); break;
             }
         };
         S.timed(kKStored, [&] {
@@ -1789,7 +1809,7 @@ template <int KIND>
 static void relax_level(Session& S, LevelData& L, const double* xin, double* xout, const double* tau, double delta,
                         double omega, double* gout = nullptr, bool cold = false)
 {
-    if (L.n_stored > 0 && L.ntiles > 0 && !S.profiling) {
+    if (L.n_stored + L.n_lat > 0 && L.ntiles > 0 && !S.profiling) {
         EGG_CK(cudaEventRecord(S.fork_ev, S.stream));
         EGG_CK(cudaStreamWaitEvent(S.side, S.fork_ev, 0));
         launch_stored<KIND>(S, L, xin, xout, tau, delta, omega, gout, S.side, cold);
@@ -1807,7 +1827,7 @@ static void sweep_once(Session& S, double* xin, double* xout, double delta, doub
 {
     launch_broadcast(S, S, xin);
     relax_level<KIND>(S, S, xin, xout, nullptr, delta, omega, nullptr, cold);
-    S.updates += S.n_interior + S.n_stored;
+    S.updates += S.n_interior + S.n_stored + S.n_lat;
 }
 
 static bool graphs_enabled()
@@ -2771,8 +2791,8 @@ int egg_b200_session_info(egg_b200_session* s, int64_t* out, int32_t n)
     return guarded([&] {
         if (!s || !out) { invalid("info: NULL argument"); }
         Session& S = *s->impl;
-        const int64_t v[11] = {S.dim,    S.M,     S.nstore,           S.n_interior + S.n_stored, S.n_interior, S.n_stored,
-                               S.nshare, S.es_ns, S.es_struct ? 1 : 0, S.prec,                    S.updates};
+        const int64_t v[11] = {S.dim,    S.M,     S.nstore,           S.n_interior + S.n_stored + S.n_lat, S.n_interior,
+                               S.n_stored + S.n_lat, S.nshare, S.es_ns, S.es_struct ? 1 : 0, S.prec,                    S.updates};
         for (int i = 0; i < n && i < 11; ++i) { out[i] = v[i]; }
     });
 }

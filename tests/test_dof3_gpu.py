@@ -4,6 +4,8 @@ NumPy-patch oracle."""
 
 from __future__ import annotations
 
+import itertools
+
 import numpy as np
 import pytest
 
@@ -40,3 +42,36 @@ def test_tile_edges_match_oracle(gpu, shape, phase, delta):
             E, _ = s.run(1, phase=phase, delta=delta, omega=0.9)
             assert np.abs(s.get_X().reshape(-1, 3) - Xo).max() <= tol
             np.testing.assert_allclose(E, Eo, rtol=1e-12 if precision == "fp64" else 1e-5)
+
+
+def _turned_cubes(perm, flips, frac=0.15, seed=2):
+    """Two 5 x 4 x 6 boxes of unit cells meeting in the plane x = 4, the second
+    one's axes permuted and reversed."""
+    a = np.stack(np.meshgrid(*[np.arange(n, dtype=float) for n in (5, 4, 6)], indexing="ij"), axis=-1)
+    b = a + np.array([4.0, 0.0, 0.0])
+    b = b.transpose(*perm, 3)[tuple(slice(None, None, -1 if f else 1) for f in flips)]
+    blocks, X = configs._dedupe([a, b])
+    free = ((X > 0) & (X < np.array([8.0, 3.0, 5.0]))).all(axis=1)
+    X = X + np.where(free[:, None], np.random.default_rng(seed).uniform(-frac, frac, X.shape), 0.0)
+    return configs.Grid("turned", 3, blocks, X, free)
+
+
+@pytest.mark.parametrize("perm", list(itertools.permutations(range(3))), ids=str)
+def test_lattice_dofs_of_turned_blocks_match_oracle(gpu, perm):
+    """The nodes of the shared face relax over a lattice table of their own
+    order, whatever way the second block is turned; a mirrored block's
+    negative dets (untangle) keep such a DOF on the general path.  One sweep
+    of fp64 sums in another order: 1e-12 of the spacing."""
+    odd = sum(perm[i] > perm[j] for i in range(3) for j in range(i + 1, 3)) % 2
+    for flips in itertools.product((0, 1), repeat=3):
+        mirrored = (odd + sum(flips)) % 2 == 1
+        phase, delta = ("untangle", 0.3) if mirrored else ("barrier", 0.0)
+        g = _turned_cubes(perm, flips)
+        Xo, Eo, _ = oracle.run3(g.X, oracle.patches_for(g.blocks, g.free, d=3), oracle.stencil_for(g.blocks, d=3), 1,
+                                phase=phase, delta=delta, omega=0.8)
+        for precision, tol in (("fp64", 1e-12), ("mixed", 1e-5)):
+            s = gpu.CppStructuredSweepSession(g.wire(), g.structured(), g.X_flat(), dim=3, precision=precision)
+            E, _ = s.run(1, phase=phase, delta=delta, omega=0.8)
+            assert np.abs(s.get_X().reshape(-1, 3) - Xo).max() <= tol
+            face = np.isclose(g.X[:, 0], 4.0, atol=0.2) & g.free
+            assert np.abs(s.get_X().reshape(-1, 3) - Xo)[face].max() <= 1e-12  # stored DOFs relax in fp64
