@@ -1148,15 +1148,16 @@ class Batch : public Session
         return {vec(E), vec(Md)};
     }
 
-    // Per-mesh positions (each flat, global node order of its mesh).
+    // Per-mesh positions (each flat, global node order of its mesh): views of
+    // one downloaded array, which lives as long as any of them.
     py::list get_X_list()
     {
         py::array_t<double> all = get_X();
-        const double* p = all.data();
+        double* p = all.mutable_data();
         py::list out;
         for (int m = 0; m < n_; ++m) {
-            std::vector<double> x(p + offs_[m] * dim_, p + offs_[m + 1] * dim_);
-            out.append(vec(x));
+            out.append(py::array_t<double>({py::ssize_t((offs_[m + 1] - offs_[m]) * dim_)},
+                                           {py::ssize_t(sizeof(double))}, p + offs_[m] * dim_, all));
         }
         return out;
     }
@@ -1164,15 +1165,24 @@ class Batch : public Session
     void set_X_list(const py::sequence& Xs)
     {
         if (int(py::len(Xs)) != n_) { throw py::value_error("set_X: one array per mesh is required"); }
-        std::vector<double> all(static_cast<size_t>(M_ * dim_));
+        std::vector<DArr> keep;
+        std::vector<const double*> ptr;
+        std::vector<int64_t> len;
         for (int m = 0; m < n_; ++m) {
             DArr a = DArr::ensure(Xs[m]);
             if (!a || int64_t(a.size()) != (offs_[m + 1] - offs_[m]) * dim_) {
                 throw py::value_error("set_X: mesh " + std::to_string(m) + " has the wrong length");
             }
-            std::copy(a.data(), a.data() + a.size(), all.begin() + offs_[m] * dim_);
+            ptr.push_back(a.data());
+            len.push_back(int64_t(a.size()));
+            keep.push_back(std::move(a));
         }
-        set_X(DArr(py::array_t<double>(int64_t(all.size()), all.data())));
+        int rc;
+        {
+            py::gil_scoped_release nogil;
+            rc = egg_b200_batch_set_X(h_.get(), ptr.data(), len.data(), n_);
+        }
+        check(rc);
     }
 
   private:

@@ -2241,18 +2241,91 @@ struct egg_b200_session {
 };
 
 
-static void ensure_xfer(Session& S)
+// Pinned staging for transfers from and to pageable memory.
+static void ensure_pin(Session& S)
 {
     const size_t n = size_t(S.M) * S.dim;
     if (!S.pin && n) {
         EGG_CK(cudaHostAlloc(reinterpret_cast<void**>(&S.pin), n * sizeof(double), cudaHostAllocDefault));
     }
+}
+
+static void ensure_xfer(Session& S)
+{
+    const size_t n = size_t(S.M) * S.dim;
     if (S.Xg.n != n) { S.Xg.alloc(n); }
     if (S.g2s_d.n != S.g2s.size()) { S.g2s_d.upload(S.g2s); }
     if (S.slot_gid_d.n != S.slot_gid.size()) { S.slot_gid_d.upload(S.slot_gid); }
     for (cudaEvent_t& e : S.xfer_ev) {
         if (!e) { EGG_CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming)); }
     }
+}
+
+static void reset_seeds(Session& S);
+
+// Positions in global node order, given as n arrays one after another, into
+// every copy of the store.  Page-locked arrays: one DMA each straight from
+// them.  The others: host thread t stages its slice of the concatenation in
+// pinned memory and queues its H2D, so the DMA of early slices overlaps the
+// staging of later ones.
+static void upload_X(Session& S, const double* const* X, const int64_t* len, int n)
+{
+    const int D = S.dim;
+    EGG_CK(cudaSetDevice(S.device));
+    ensure_xfer(S);
+    std::vector<size_t> at(size_t(n) + 1, 0);
+    std::vector<char> pinned(size_t(n), 0);
+    size_t staged = 0;
+    for (int m = 0; m < n; ++m) {
+        at[size_t(m) + 1] = at[size_t(m)] + size_t(len[m]);
+        if (!len[m]) { continue; }
+        cudaPointerAttributes attr {};
+        pinned[size_t(m)] = cudaPointerGetAttributes(&attr, X[m]) == cudaSuccess && attr.type == cudaMemoryTypeHost;
+        cudaGetLastError();
+        if (pinned[size_t(m)]) {
+            EGG_CK(cudaMemcpyAsync(S.Xg.p + at[size_t(m)], X[m], size_t(len[m]) * sizeof(double),
+                                   cudaMemcpyHostToDevice, S.stream));
+        } else {
+            staged += size_t(len[m]);
+        }
+    }
+    if (staged) {
+        ensure_pin(S);
+        const size_t total = at[size_t(n)];
+        const int T = copy_threads(staged * sizeof(double));
+        cudaError_t err[kMaxCopyThreads] = {};
+        run_slices(T, [&](int t) {
+            const size_t a = slice_begin(total, t, T), b = slice_begin(total, t + 1, T);
+            err[t] = cudaSetDevice(S.device);
+            size_t m = size_t(std::upper_bound(at.begin(), at.end(), a) - at.begin()) - 1;
+            for (; m < size_t(n) && at[m] < b; ++m) {
+                const size_t lo = std::max(a, at[m]), hi = std::min(b, at[m + 1]);
+                if (pinned[m] || hi <= lo || err[t] != cudaSuccess) { continue; }
+                std::memcpy(S.pin + lo, X[m] + (lo - at[m]), (hi - lo) * sizeof(double));
+                err[t] = cudaMemcpyAsync(S.Xg.p + lo, S.pin + lo, (hi - lo) * sizeof(double), cudaMemcpyHostToDevice,
+                                         S.stream);
+            }
+        });
+        for (int t = 0; t < T; ++t) { EGG_CK(err[t]); }
+    }
+    if (S.nstore) {
+        if (D == 2) {
+            gather_global_kernel<2><<<remap_grid(S.nstore), 256, 0, S.stream>>>(S.Xg.p, S.slot_gid_d.p, S.nstore,
+                                                                             S.X(S.cur));
+        } else {
+            gather_global_kernel<3><<<remap_grid(S.nstore), 256, 0, S.stream>>>(S.Xg.p, S.slot_gid_d.p, S.nstore,
+                                                                             S.X(S.cur));
+        }
+        EGG_CK(cudaGetLastError());
+        ++S.launches;
+    }
+    for (size_t j = 0; j < S.nb_gid.size(); ++j) {
+        const size_t e = size_t(S.nb_gid[j]) * size_t(D);
+        const size_t m = size_t(std::upper_bound(at.begin(), at.end(), e) - at.begin()) - 1;
+        for (int k = 0; k < D; ++k) { S.nb_val[j * D + k] = X[m][e - at[m] + size_t(k)]; }
+    }
+    reset_seeds(S);  // new positions: B-spline projections start cold
+    S.sync();
 }
 
 // The B-spline seeds after a position reset: NaN (the next projection seeds
@@ -2708,6 +2781,7 @@ int egg_b200_session_get_X(egg_b200_session* s, double* X, int64_t len)
         // t waits for slice t only, so the copy-out of early slices overlaps
         // the DMA.
         const int T = pinned ? 0 : copy_threads(n * sizeof(double));
+        if (T) { ensure_pin(S); }
         for (int t = 0; t < T; ++t) {
             const size_t a = slice_begin(n, t, T), b = slice_begin(n, t + 1, T);
             if (b > a) {
@@ -2738,51 +2812,25 @@ int egg_b200_session_set_X(egg_b200_session* s, const double* X, int64_t len)
     return guarded([&] {
         if (!s || !X) { invalid("set_X: NULL argument"); }
         Session& S = *s->impl;
-        const int D = S.dim;
-        if (len != S.M * D) { invalid("set_X: input length != num_nodes*dim"); }
-        EGG_CK(cudaSetDevice(S.device));
-        ensure_xfer(S);
-        const size_t n = size_t(len);
-        // Page-locked input: one DMA straight from it.  Otherwise host thread
-        // t stages slice t in pinned memory and queues its H2D, so the DMA of
-        // early slices overlaps the staging of later ones.
-        cudaPointerAttributes attr {};
-        const bool pinned = cudaPointerGetAttributes(&attr, X) == cudaSuccess && attr.type == cudaMemoryTypeHost;
-        cudaGetLastError();
-        if (pinned && n) {
-            EGG_CK(cudaMemcpyAsync(S.Xg.p, X, n * sizeof(double), cudaMemcpyHostToDevice, S.stream));
-        }
-        const int T = pinned ? 0 : copy_threads(n * sizeof(double));
-        cudaError_t err[kMaxCopyThreads] = {};
-        if (T > 0) {
-            run_slices(T, [&](int t) {
-                const size_t a = slice_begin(n, t, T), b = slice_begin(n, t + 1, T);
-                if (b == a) { return; }
-                std::memcpy(S.pin + a, X + a, (b - a) * sizeof(double));
-                err[t] = cudaSetDevice(S.device);
-                if (err[t] == cudaSuccess) {
-                    err[t] = cudaMemcpyAsync(S.Xg.p + a, S.pin + a, (b - a) * sizeof(double), cudaMemcpyHostToDevice,
-                                             S.stream);
-                }
-            });
-        }
-        for (int t = 0; t < T; ++t) { EGG_CK(err[t]); }
-        if (S.nstore) {
-            if (D == 2) {
-                gather_global_kernel<2><<<remap_grid(S.nstore), 256, 0, S.stream>>>(S.Xg.p, S.slot_gid_d.p, S.nstore,
-                                                                                 S.X(S.cur));
-            } else {
-                gather_global_kernel<3><<<remap_grid(S.nstore), 256, 0, S.stream>>>(S.Xg.p, S.slot_gid_d.p, S.nstore,
-                                                                                 S.X(S.cur));
+        if (len != S.M * S.dim) { invalid("set_X: input length != num_nodes*dim"); }
+        upload_X(S, &X, &len, 1);
+    });
+}
+
+int egg_b200_batch_set_X(egg_b200_session* s, const double* const* X, const int64_t* len, int32_t n_meshes)
+{
+    return guarded([&] {
+        if (!s || !X || !len) { invalid("batch_set_X: NULL argument"); }
+        Session& S = *s->impl;
+        if (S.n_seg <= 0) { invalid("batch_set_X: not a batch session"); }
+        if (n_meshes != S.n_seg) { invalid("batch_set_X: one array per mesh is required"); }
+        for (int32_t m = 0; m < n_meshes; ++m) {
+            if (len[m] != (S.mesh_node_off[size_t(m) + 1] - S.mesh_node_off[size_t(m)]) * S.dim) {
+                invalid("batch_set_X: mesh " + std::to_string(m) + " has the wrong length");
             }
-            EGG_CK(cudaGetLastError());
-            ++S.launches;
+            if (!X[m] && len[m]) { invalid("batch_set_X: NULL array"); }
         }
-        for (size_t j = 0; j < S.nb_gid.size(); ++j) {
-            for (int k = 0; k < D; ++k) { S.nb_val[j * D + k] = X[S.nb_gid[j] * D + k]; }
-        }
-        reset_seeds(S);  // new positions: B-spline projections start cold
-        S.sync();
+        upload_X(S, X, len, n_meshes);
     });
 }
 

@@ -499,6 +499,10 @@ int egg_b200_session_get_X(egg_b200_session* s, double* X, int64_t len);
  * Replaces SweepDeviceContextT::upload_X (src/sweep.hpp:552-557). */
 int egg_b200_session_set_X(egg_b200_session* s, const double* X, int64_t len);
 
+/* set_X of a batch session from one array per mesh (len[m] reals each, mesh
+ * m's own node order), without a concatenated copy on the host. */
+int egg_b200_batch_set_X(egg_b200_session* s, const double* const* X, const int64_t* len, int32_t n_meshes);
+
 /* Session facts: [0] dim, [1] global nodes, [2] packed store nodes, [3] moving
  * DOFs, [4] structured-interior DOFs, [5] stored-patch DOFs, [6] owner->copy
  * entries, [7] energy samples, [8] structured energy stencil (0/1),
