@@ -20,6 +20,8 @@
 
 #include "kernels3d.cuh"
 
+#include <cooperative_groups.h>
+
 namespace egg_b200
 {
 
@@ -154,11 +156,10 @@ __global__ void ctl_eval_kernel(CtlTables T, int64_t total_nodes, const double* 
 // C_dir[lattice] = v[free] on free controls, 0 elsewhere.
 template <int D>
 __global__ void ctl_scatter_kernel(CtlTables T, int64_t total_ctrl, const double* __restrict__ v,
-                                   double* __restrict__ Cdir, const PcgState* __restrict__ st)
+                                   double* __restrict__ Cdir)
 {
     for (int64_t g = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; g < total_ctrl;
          g += int64_t(gridDim.x) * blockDim.x) {
-        if (st && st[net_of(T.ctrl_pfx, T.n_nets, g)].done) { continue; }
         const int32_t f = T.free_of[g];
 #pragma unroll
         for (int c = 0; c < D; ++c) { Cdir[g * D + c] = f >= 0 ? v[int64_t(f) * D + c] : 0.0; }
@@ -216,6 +217,29 @@ __global__ void ctl_dir_scatter_kernel(CtlTables T, const SoftTerm* __restrict__
     }
 }
 
+// Hessian-vector product of the 2D metric, from its closed form (metric.cuh)
+// without the 4 x 4 Hessian: with P dT = cof(dT) and D' = cof : dT,
+//   H dT = 2 f dT + 2 f' (T D' + cof (T : dT)) + s f'' D' cof + s f' P dT.
+template <int KIND> __device__ __forceinline__ void mu2_hvp(const double t[4], const double dt[4], double hv[4])
+{
+    const double cof[4] = {t[3], -t[2], -t[1], t[0]}, pd[4] = {dt[3], -dt[2], -dt[1], dt[0]};
+    const double D = det2(t), s = t[0] * t[0] + t[1] * t[1] + t[2] * t[2] + t[3] * t[3];
+    const ScaleFn<double> sf = shape_scale(D);
+    const double Dd = cof[0] * dt[0] + cof[1] * dt[1] + cof[2] * dt[2] + cof[3] * dt[3];
+    const double td = t[0] * dt[0] + t[1] * dt[1] + t[2] * dt[2] + t[3] * dt[3];
+    const double a = 2.0 * sf.fp * Dd, b = 2.0 * sf.fp * td + s * sf.fpp * Dd, c = s * sf.fp;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { hv[i] = 2.0 * sf.f * dt[i] + a * t[i] + b * cof[i] + c * pd[i]; }
+    if constexpr (KIND == kShapeSize) {  // mu = m^2 - 1 + (D - 1)^2, m = s f
+        const double m = s * sf.f, md = 2.0 * sf.f * td + c * Dd, dm1 = D - 1.0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const double g = 2.0 * sf.f * t[i] + c * cof[i];
+            hv[i] = 2.0 * md * g + 2.0 * m * hv[i] + 2.0 * Dd * cof[i] + 2.0 * dm1 * pd[i];
+        }
+    }
+}
+
 // Per-node gradient / Hessian-vector product / contracted Hessian over the
 // block's canonical cell stencil (see the file comment).
 template <int D, int KIND, int MODE>
@@ -238,19 +262,19 @@ __global__ void ctl_node_kernel(CtlTables T, int64_t total_nodes, EnergyStructur
         double acc[OUTW];
 #pragma unroll
         for (int i = 0; i < OUTW; ++i) { acc[i] = 0.0; }
-        // cells around the node in ascending cell order
+        // cells around the node in ascending cell order (unrolled in 2D: which
+        // samples move the node, and in what role, is then known at compile time)
+#pragma unroll(D == 2 ? NC : 1)
         for (int cc = 0; cc < NC; ++cc) {
             int cl[3] = {L[0] - 1 + ((cc >> (D - 1)) & 1), L[1] - 1 + ((cc >> (D - 2)) & 1),
                          D == 3 ? L[2] - 1 + (cc & 1) : 0};
             if (cl[0] < 0 || cl[0] > n0 - 2 || cl[1] < 0 || cl[1] > n1 - 2) { continue; }
             if (D == 3 && (cl[2] < 0 || cl[2] > n2 - 2)) { continue; }
-            // node's corner index inside the cell (axis 0 most significant)
-            int q = 0;
-#pragma unroll
-            for (int k = 0; k < D; ++k) { q = (q << 1) | (L[k] - cl[k]); }
+            const int q = cc ^ (NC - 1);  // node's corner index inside the cell (axis 0 most significant)
             const int64_t lc = (int64_t(cl[0]) * c1 + cl[1]) * c2 + (D == 3 ? cl[2] : 0);
             const int64_t cell = n.cell_off + lc;
             const int64_t base = n.node_off + (int64_t(cl[0]) * n1 + cl[1]) * n2 + (D == 3 ? cl[2] : 0);
+#pragma unroll(D == 2 ? NC : 1)
             for (int b = 0; b < NC; ++b) {
                 int role = -1;
                 if (q == b) {
@@ -280,7 +304,7 @@ __global__ void ctl_node_kernel(CtlTables T, int64_t total_nodes, EnergyStructur
                     double t[4], detA;
                     assemble_T(X2[sc], X2[sa], X2[sb], s[0], s[1], w, t, detA);
                     double mu, gT[4], H[16];
-                    mu_eval<double>(KIND, t, 0.0, mu, gT, H);
+                    if constexpr (MODE != kCtlHvp) { mu_eval<double>(KIND, t, 0.0, mu, gT, H); }
                     if constexpr (MODE == kCtlGrad) {
 #pragma unroll
                         for (int i = 0; i < 2; ++i) { acc[i] += wt * (gT[2 * i] * v[0] + gT[2 * i + 1] * v[1]); }
@@ -294,10 +318,7 @@ __global__ void ctl_node_kernel(CtlTables T, int64_t total_nodes, EnergyStructur
                         double dt[4], dd;
                         assemble_T(dc, da, db, s[0], s[1], w, dt, dd);
                         double hv[4];
-#pragma unroll
-                        for (int a = 0; a < 4; ++a) {
-                            hv[a] = H[4 * a] * dt[0] + H[4 * a + 1] * dt[1] + H[4 * a + 2] * dt[2] + H[4 * a + 3] * dt[3];
-                        }
+                        mu2_hvp<KIND>(t, dt, hv);
 #pragma unroll
                         for (int i = 0; i < 2; ++i) { acc[i] += wt * (hv[2 * i] * v[0] + hv[2 * i + 1] * v[1]); }
                     } else {
@@ -382,15 +403,22 @@ __device__ __forceinline__ Support<D> support_of(const CtlTables& T, const CtlNe
 }
 
 // Free-control pullback out_f = sum_{n in supp(f)} w_n y_n (+ lam v_f), or the
-// Jacobi block P_f = sum w_n^2 h_n (PRECOND).
-template <int D, bool PRECOND>
+// Jacobi block P_f = sum w_n^2 h_n (PRECOND).  A control's support is a box of
+// a few hundred nodes.  WARP: its warp's lanes stride over the box, consecutive
+// lanes along the last axis, and add up by butterfly; otherwise one thread
+// adds in the reference's order, a serial chain of loads (257^2 block, 64^2
+// net: 53 us against 7.5).  Topologies and walled nets keep the serial
+// order: their frames amplify a last bit (a sphere's chart near its pole,
+// 7e7-fold), and their nets are small.
+template <int D, bool PRECOND, bool WARP>
 __global__ void ctl_pullback_kernel(CtlTables T, int64_t total_free, const double* __restrict__ y,
                                     double* __restrict__ out, const double* __restrict__ v,
                                     const PcgState* __restrict__ st)
 {
-    constexpr int W = PRECOND ? D * D : D;
-    for (int64_t g = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; g < total_free;
-         g += int64_t(gridDim.x) * blockDim.x) {
+    constexpr int W = PRECOND ? D * D : D, G = WARP ? 32 : 1;
+    const int lane = threadIdx.x & (G - 1);
+    const int64_t ngroup = (int64_t(gridDim.x) * blockDim.x) / G;
+    for (int64_t g = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) / G; g < total_free; g += ngroup) {
         const int ni = net_of(T.free_pfx, T.n_nets, g);
         if (st && !PRECOND && st[ni].done) { continue; }
         const CtlNet n = T.nets[ni];
@@ -401,177 +429,256 @@ __global__ void ctl_pullback_kernel(CtlTables T, int64_t total_free, const doubl
         double acc[W];
 #pragma unroll
         for (int i = 0; i < W; ++i) { acc[i] = 0.0; }
-        const int l2 = D == 3 ? sp.len[2] : 1;
-        for (int t0 = 0; t0 < sp.len[0]; ++t0) {
-            for (int t1 = 0; t1 < sp.len[1]; ++t1) {
-                for (int t2 = 0; t2 < l2; ++t2) {
-                    double w = 1.0 * sp.w[0][t0] * sp.w[1][t1];
-                    int64_t nd = int64_t(sp.node[0][t0]) * n.node_shape[1] + sp.node[1][t1];
-                    if (D == 3) {
-                        w *= sp.w[2][t2];
-                        nd = nd * n.node_shape[2] + sp.node[2][t2];
-                    }
-                    const int64_t gn = n.n_off + nd;
-                    if (PRECOND) {
-                        const double w2 = w * w;
-#pragma unroll
-                        for (int i = 0; i < W; ++i) { acc[i] += w2 * y[gn * W + i]; }
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < W; ++i) { acc[i] += w * y[gn * W + i]; }
-                    }
-                }
+        const int ll = sp.len[D - 1], l1 = D == 3 ? sp.len[1] : 1;
+        const int rows = sp.len[0] * l1;
+        for (int e = lane; e < rows * ll; e += G) {
+            const int row = e / ll, tl = e - row * ll;
+            const int t0 = D == 3 ? row / l1 : row;
+            double w = sp.w[0][t0];
+            int64_t nd = sp.node[0][t0];
+            if constexpr (D == 3) {
+                w *= sp.w[1][row - t0 * l1];
+                nd = nd * n.node_shape[1] + sp.node[1][row - t0 * l1];
             }
+            w *= sp.w[D - 1][tl];
+            nd = nd * n.node_shape[D - 1] + sp.node[D - 1][tl];
+            const int64_t gn = n.n_off + nd;
+            if (PRECOND) { w *= w; }
+#pragma unroll
+            for (int i = 0; i < W; ++i) { acc[i] += w * y[gn * W + i]; }
         }
+#pragma unroll
+        for (int i = 0; i < W; ++i) { acc[i] = group_sum<G>(acc[i]); }
         if (!PRECOND && st && st[ni].lam > 0.0) {
 #pragma unroll
             for (int i = 0; i < W; ++i) { acc[i] += st[ni].lam * v[g * W + i]; }
         }
+        if (lane == 0) {
 #pragma unroll
-        for (int i = 0; i < W; ++i) { out[g * W + i] = acc[i]; }
-    }
-}
-
-// z_f = (P_f + lam I)^{-1} r_f with the Newton-solve fallbacks (src/solve.hpp).
-template <int D>
-__global__ void ctl_precond_apply_kernel(CtlTables T, int64_t total_free, const double* __restrict__ prec,
-                                         const double* __restrict__ r, double* __restrict__ z,
-                                         const PcgState* __restrict__ st)
-{
-    for (int64_t g = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; g < total_free;
-         g += int64_t(gridDim.x) * blockDim.x) {
-        const int ni = net_of(T.free_pfx, T.n_nets, g);
-        if (st[ni].done) { continue; }
-        const double lam = st[ni].lam;
-        const double* P = prec + g * D * D;
-        double rhs[3], x[3];
-#pragma unroll
-        for (int i = 0; i < D; ++i) { rhs[i] = -r[g * D + i]; }
-        if (D == 2) {
-            const double H[4] = {P[0] + lam, P[1], P[2], P[3] + lam};
-            solve2<double>(H, rhs, x);
-        } else {
-            const double h6[6] = {P[0] + lam, P[1], P[2], P[4] + lam, P[5], P[8] + lam};
-            solve3<double>(h6, rhs, x);
+            for (int i = 0; i < W; ++i) { out[g * W + i] = acc[i]; }
         }
-#pragma unroll
-        for (int i = 0; i < D; ++i) { z[g * D + i] = x[i]; }
     }
 }
 
-// Per-net reductions over the stacked free vector (one CTA row per net, fixed
-// order, compensated), with the PCG scalar step of the reduction folded into
-// thread 0 (src/control_solve.hpp:761-819):
+// z = (P_f + lam I)^{-1} r with the Newton-solve fallbacks (src/solve.hpp).
+template <int D> __device__ __forceinline__ void ctl_precond(const double* P, double lam, const double r[D], double z[D])
+{
+    double rhs[3], x[3];
+#pragma unroll
+    for (int i = 0; i < D; ++i) { rhs[i] = -r[i]; }
+    if constexpr (D == 2) {
+        const double H[4] = {P[0] + lam, P[1], P[2], P[3] + lam};
+        solve2<double>(H, rhs, x);
+    } else {
+        const double h6[6] = {P[0] + lam, P[1], P[2], P[4] + lam, P[5], P[8] + lam};
+        solve3<double>(h6, rhs, x);
+    }
+#pragma unroll
+    for (int i = 0; i < D; ++i) { z[i] = x[i]; }
+}
+
+// Per-net reductions over the stacked free vector (one CTA per net, fixed
+// order, compensated).
 enum {
-    kRedStore = 0,   // out[net] = x . y
-    kRedAmax,        // out[net] = max |x|
-    kRedTrace,       // out[net] = sum of diagonals of the D x D blocks of x
-    kRedInit,        // r.r:   b_norm2, stop2 = rtol^2 b, r_norm2; done when b == 0
-    kRedRz0,         // r.z:   rz
-    kRedPap,         // p.Ap:  stop on non-positive curvature, else alpha = rz / pAp
-    kRedRr,          // r.r:   r_norm2; stop when <= stop2 (its = it + 1)
-    kRedRz,          // r.z:   beta = rz_new / rz, rz = rz_new, ++it, stop at max_iter
+    kRedAmax = 0,  // out[net] = max |x|
+    kRedTrace,     // out[net] = sum of diagonals of the D x D blocks of x
 };
 
 template <int D, int OP>
-__global__ void ctl_reduce_kernel(CtlTables T, const double* __restrict__ x, const double* __restrict__ y,
-                                  double* __restrict__ out, PcgState* __restrict__ st, double rtol)
+__global__ void ctl_reduce_kernel(CtlTables T, const double* __restrict__ x, double* __restrict__ out)
 {
     const int ni = blockIdx.x;
-    const bool skip = (OP >= kRedPap) && st[ni].done;
-    if (skip) { return; }  // uniform across the CTA
-    const int64_t W = OP == kRedTrace ? D * D : D;
-    const int64_t lo = T.free_pfx[ni] * W, hi = T.free_pfx[ni + 1] * W;
     Comp acc {0.0, 0.0};
     double mx = 0.0;
-    for (int64_t i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-        if (OP == kRedAmax) {
-            mx = fmax(mx, fabs(x[i]));
-        } else if (OP == kRedTrace) {
-            const int64_t e = i - lo;
-            if ((e % (D * D)) % (D + 1) == 0) { comp_add(acc, x[i]); }
-        } else {
-            comp_add(acc, x[i] * y[i]);
+    for (int64_t g = T.free_pfx[ni] + threadIdx.x; g < T.free_pfx[ni + 1]; g += blockDim.x) {
+#pragma unroll
+        for (int i = 0; i < D; ++i) {
+            if (OP == kRedAmax) {
+                mx = fmax(mx, fabs(x[g * D + i]));
+            } else {
+                comp_add(acc, x[g * D * D + i * (D + 1)]);
+            }
         }
     }
     // max via the min slot of the shared reducer
     double mn = -mx;
     if (!block_reduce(acc, mn)) { return; }
-    const double v = OP == kRedAmax ? -mn : acc.s + acc.c;
-    PcgState& s = st[ni];
-    switch (OP) {
-    case kRedStore:
-    case kRedAmax:
-    case kRedTrace: out[ni] = v; break;
-    case kRedInit:
-        s.b_norm2 = v;
-        s.r_norm2 = v;
-        {
-            // rtol < 0: the per-net relative tolerance was preloaded into stop2
-            const double rt = rtol >= 0.0 ? rtol : s.stop2;
-            s.stop2 = rt * rt * v;
-        }
-        s.it = 0;
-        s.its = 0;
-        s.done = (v == 0.0 || !s.active || s.max_iter <= 0) ? 1 : 0;
-        break;
-    case kRedRz0: s.rz = v; break;
-    case kRedPap:
-        if (!(v > 0.0)) {
-            s.its = s.it;
-            s.done = 1;
-        } else {
-            s.alpha = s.rz / v;
-        }
-        break;
-    case kRedRr:
-        s.r_norm2 = v;
-        if (v <= s.stop2) {
-            s.its = s.it + 1;
-            s.done = 1;
-        }
-        break;
-    case kRedRz:
-        s.beta = v / s.rz;
-        s.rz = v;
-        s.it += 1;
-        if (s.it >= s.max_iter) {
-            s.its = s.it;
-            s.done = 1;
-        }
-        break;
-    }
+    out[ni] = OP == kRedAmax ? -mn : acc.s + acc.c;
 }
 
-// PCG vector updates over the stacked free vector (skipping finished nets).
-enum { kVecInit = 0, kVecAxpy2, kVecXpay, kVecCopy };
+// The vector part of a PCG iteration (src/control_solve.hpp:761-819): dot
+// products, updates and preconditioner in one launch, a cluster of kCgCluster
+// CTAs per net.  Each dot product is reduced per CTA, exchanged through
+// distributed shared memory and added in rank order, so every thread holds the
+// same total and takes the same decisions.  A CG iteration on a 64^2 net took
+// 10 launches and 105 us (three one-CTA reductions among them), in one CTA of
+// 512 threads 4 launches and 44 us, with the cluster 31.
+constexpr int kCgCluster = 8;
+constexpr int kCgThreads = 512;
 
-template <int D, int OP>
-__global__ void ctl_vec_kernel(CtlTables T, int64_t total_free, double* __restrict__ a, double* __restrict__ b,
-                               const double* __restrict__ c, const double* __restrict__ d,
-                               const PcgState* __restrict__ st)
+struct CgShared {
+    Comp part[3];
+    double total[3];
+};
+
+// The cluster's totals of acc[0 .. N), exchange slots first .. first + N.
+template <int N>
+__device__ __forceinline__ void ctl_cluster_total(CgShared& sh, int first, const Comp (&acc)[N], double (&out)[N])
 {
-    for (int64_t g = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; g < total_free;
-         g += int64_t(gridDim.x) * blockDim.x) {
-        const int ni = net_of(T.free_pfx, T.n_nets, g);
-        if (OP == kVecInit ? !st[ni].active : st[ni].done) { continue; }
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        Comp a = acc[k];
+        double mn = 0.0;
+        if (block_reduce(a, mn)) { sh.part[first + k] = a; }
+        __syncthreads();  // the reducer's storage is free again
+    }
+    cl.sync();
+    if (threadIdx.x < N) {
+        Comp t {0.0, 0.0};
+        for (unsigned q = 0; q < unsigned(kCgCluster); ++q) {
+            t = comp_merge(t, cl.map_shared_rank(&sh, q)->part[first + threadIdx.x]);
+        }
+        sh.total[first + threadIdx.x] = t.s + t.c;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < N; ++k) { out[k] = sh.total[first + k]; }
+}
+
+// Start: dC = 0, r = -G, z = P^{-1} r, p = z (also scattered to the lattice,
+// Cdir), b.b, r.z; the net's relative tolerance arrives in stop2.
+template <int D>
+__global__ void __cluster_dims__(kCgCluster, 1, 1) __launch_bounds__(kCgThreads)
+  ctl_cg_start_kernel(CtlTables T, const double* __restrict__ G, const double* __restrict__ prec,
+                      double* __restrict__ dC, double* __restrict__ r, double* __restrict__ p,
+                      double* __restrict__ Cdir, PcgState* __restrict__ st)
+{
+    __shared__ CgShared sh;
+    const int ni = blockIdx.x / kCgCluster, rank = blockIdx.x % kCgCluster;
+    PcgState& s = st[ni];
+    const bool lead = rank == 0 && threadIdx.x == 0;
+    if (!s.active) {  // uniform across the cluster
+        if (lead) { s.done = 1; }
+        return;
+    }
+    const double lam = s.lam, tol = s.stop2;
+    const int max_iter = s.max_iter;
+    const int64_t c_off = T.nets[ni].c_off;
+    Comp acc[2] = {{0.0, 0.0}, {0.0, 0.0}};
+    for (int64_t g = T.free_pfx[ni] + rank * kCgThreads + threadIdx.x; g < T.free_pfx[ni + 1];
+         g += kCgCluster * kCgThreads) {
+        double rr[D], z[D];
+#pragma unroll
+        for (int i = 0; i < D; ++i) { rr[i] = -G[g * D + i]; }
+        ctl_precond<D>(prec + g * D * D, lam, rr, z);
+        const int64_t ci = c_off + T.free_idx[g];
 #pragma unroll
         for (int i = 0; i < D; ++i) {
-            const int64_t e = g * D + i;
-            if (OP == kVecInit) {          // a = dC = 0, b = r = -G (c)
-                a[e] = 0.0;
-                b[e] = -c[e];
-            } else if (OP == kVecAxpy2) {  // a = dC += alpha p (c); b = r -= alpha Ap (d)
-                const double al = st[ni].alpha;
-                a[e] += al * c[e];
-                b[e] -= al * d[e];
-            } else if (OP == kVecXpay) {   // a = p = z (c) + beta p
-                a[e] = c[e] + st[ni].beta * a[e];
-            } else {                       // a = p = z (c)
-                a[e] = c[e];
+            dC[g * D + i] = 0.0;
+            r[g * D + i] = rr[i];
+            p[g * D + i] = z[i];
+            Cdir[ci * D + i] = z[i];
+            comp_add(acc[0], rr[i] * rr[i]);
+            comp_add(acc[1], rr[i] * z[i]);
+        }
+    }
+    double t[2];
+    ctl_cluster_total<2>(sh, 0, acc, t);
+    if (lead) {
+        s.b_norm2 = t[0];
+        s.r_norm2 = t[0];
+        s.stop2 = tol * tol * t[0];
+        s.rz = t[1];
+        s.it = 0;
+        s.its = 0;
+        s.done = (t[0] == 0.0 || max_iter <= 0) ? 1 : 0;
+    }
+    cooperative_groups::this_cluster().sync();  // no CTA leaves while its partials are read
+}
+
+// One iteration after Ap: p.Ap (stop on non-positive curvature), dC += alpha p,
+// r -= alpha Ap, r.r (stop at stop2), z = P^{-1} r, r.z, p = z + beta p.
+template <int D>
+__global__ void __cluster_dims__(kCgCluster, 1, 1) __launch_bounds__(kCgThreads)
+  ctl_cg_step_kernel(CtlTables T, const double* __restrict__ prec, const double* __restrict__ Ap,
+                     double* __restrict__ dC, double* __restrict__ r, double* __restrict__ z, double* __restrict__ p,
+                     double* __restrict__ Cdir, PcgState* __restrict__ st)
+{
+    __shared__ CgShared sh;
+    const int ni = blockIdx.x / kCgCluster, rank = blockIdx.x % kCgCluster;
+    PcgState& s = st[ni];
+    if (s.done) { return; }  // uniform: the lead thread writes it past two cluster barriers
+    const bool lead = rank == 0 && threadIdx.x == 0;
+    const double rz_old = s.rz, lam = s.lam, stop2 = s.stop2;
+    const int it = s.it, max_iter = s.max_iter;
+    const int64_t lo = T.free_pfx[ni] + rank * kCgThreads + threadIdx.x, hi = T.free_pfx[ni + 1];
+    constexpr int64_t step = kCgCluster * kCgThreads;
+    Comp pp[1] = {{0.0, 0.0}};
+    for (int64_t g = lo; g < hi; g += step) {
+#pragma unroll
+        for (int i = 0; i < D; ++i) { comp_add(pp[0], p[g * D + i] * Ap[g * D + i]); }
+    }
+    double pap[1];
+    ctl_cluster_total<1>(sh, 0, pp, pap);
+    const bool down = !(pap[0] > 0.0);
+    const double alpha = rz_old / pap[0];
+    Comp acc[2] = {{0.0, 0.0}, {0.0, 0.0}};
+    if (!down) {
+        for (int64_t g = lo; g < hi; g += step) {
+            double rv[D], zv[D];
+#pragma unroll
+            for (int i = 0; i < D; ++i) {
+                const int64_t e = g * D + i;
+                dC[e] += alpha * p[e];
+                rv[i] = r[e] - alpha * Ap[e];
+                r[e] = rv[i];
+                comp_add(acc[0], rv[i] * rv[i]);
+            }
+            ctl_precond<D>(prec + g * D * D, lam, rv, zv);
+#pragma unroll
+            for (int i = 0; i < D; ++i) {
+                z[g * D + i] = zv[i];
+                comp_add(acc[1], rv[i] * zv[i]);
             }
         }
     }
+    double t[2];
+    ctl_cluster_total<2>(sh, 1, acc, t);
+    const bool small = t[0] <= stop2, last = it + 1 >= max_iter;
+    if (lead) {
+        if (down) {
+            s.its = it;
+            s.done = 1;
+        } else {
+            s.alpha = alpha;
+            s.r_norm2 = t[0];
+            if (!small) {
+                s.beta = t[1] / rz_old;
+                s.rz = t[1];
+                s.it = it + 1;
+            }
+            if (small || last) {
+                s.its = it + 1;
+                s.done = 1;
+            }
+        }
+    }
+    if (!(down || small || last)) {
+        const double beta = t[1] / rz_old;
+        const int64_t c_off = T.nets[ni].c_off;
+        for (int64_t g = lo; g < hi; g += step) {
+            const int64_t ci = c_off + T.free_idx[g];
+#pragma unroll
+            for (int i = 0; i < D; ++i) {
+                const double v = z[g * D + i] + beta * p[g * D + i];
+                p[g * D + i] = v;
+                Cdir[ci * D + i] = v;
+            }
+        }
+    }
+    cooperative_groups::this_cluster().sync();  // no CTA leaves while its partials are read
 }
 
 // Trial / commit on the net nodes: out[slot] = X[slot] + alpha[net] corr[node]
