@@ -29,11 +29,14 @@ struct BlockInfo {
     int32_t pad;
 };
 
-struct Tile2 {
-    int32_t block;
-    int32_t i0;  // first DOF row (logical, >= 1)
-    int32_t j0;  // first DOF column
-    int32_t pad;
+// A tile of structured-interior DOFs with its block's data, so that a CTA
+// starts on one load instead of two dependent ones.
+struct __align__(16) Tile2 {
+    int64_t off;     // first node slot of the block
+    int32_t n0, n1;  // the block's node counts
+    int32_t i0;      // first DOF row (logical, >= 1)
+    int32_t j0;      // first DOF column
+    int32_t pad[2];
 };
 
 // Relative threshold of the fp64 guard in mixed precision: a sample whose
@@ -59,31 +62,6 @@ __device__ __forceinline__ void sample_full_c(C ax, C bx, C ay, C by, C delta, S
     const C t[4] = {ax, bx, ay, by};
     mu_eval<C>(KIND, t, delta, o.mu, o.g, o.H);
     o.det = det2(t);
-}
-
-// Full per-sample evaluation from fp64 edge vectors, in working precision C
-// (fp64 re-evaluation for near-degenerate samples when C = float).
-template <int KIND, class C>
-__device__ __forceinline__ void sample_full(double ax, double bx, double ay, double by, double delta,
-                                            SampleOut<C>& o)
-{
-    if constexpr (std::is_same_v<C, double>) {
-        sample_full_c<KIND, double>(ax, bx, ay, by, delta, o);
-    } else {
-        const float fax = float(ax), fbx = float(bx), fay = float(ay), fby = float(by);
-        const float d = fax * fby - fbx * fay;
-        const float n0 = fax * fax + fay * fay, n1 = fbx * fbx + fby * fby;
-        if (d * d < float(kGuard * kGuard) * n0 * n1) {
-            SampleOut<double> od;
-            sample_full_c<KIND, double>(ax, bx, ay, by, delta, od);
-            o.mu = float(od.mu);
-            o.det = float(od.det);
-            for (int i = 0; i < 4; ++i) { o.g[i] = float(od.g[i]); }
-            for (int i = 0; i < 16; ++i) { o.H[i] = float(od.H[i]); }
-        } else {
-            sample_full_c<KIND, float>(fax, fbx, fay, fby, float(delta), o);
-        }
-    }
 }
 
 // Value + det only (line-search trials), working precision C with fp64 guard.
@@ -169,34 +147,6 @@ __device__ __forceinline__ void sample_roles_c(C a, C b, C c, C d, C s0, C s1, C
     o.r[0][4] = h22 + h33 + C(2) * ss * h23;
 }
 
-// Role contributions from fp64 edge vectors in working precision C, with the
-// fp64 re-evaluation of near-degenerate samples when C = float.
-template <int KIND, class C>
-__device__ __forceinline__ void sample_roles(double ax, double bx, double ay, double by, double s0, double s1,
-                                             double delta, RoleOut<C>& o)
-{
-    if constexpr (std::is_same_v<C, double>) {
-        sample_roles_c<KIND, double>(ax, bx, ay, by, s0, s1, delta, o);
-    } else {
-        const float fax = float(ax), fbx = float(bx), fay = float(ay), fby = float(by);
-        const float d = fax * fby - fbx * fay;
-        const float n0 = fax * fax + fay * fay, n1 = fbx * fbx + fby * fby;
-        if (d * d < float(kGuard * kGuard) * n0 * n1) {
-            RoleOut<double> od;
-            sample_roles_c<KIND, double>(ax, bx, ay, by, s0, s1, delta, od);
-            o.mu = float(od.mu);
-            o.det = float(od.det);
-#pragma unroll
-            for (int r = 0; r < 3; ++r) {
-#pragma unroll
-                for (int q = 0; q < 5; ++q) { o.r[r][q] = float(od.r[r][q]); }
-            }
-        } else {
-            sample_roles_c<KIND, float>(fax, fbx, fay, fby, float(s0), float(s1), float(delta), o);
-        }
-    }
-}
-
 // ---------------------------------------------------------------------------
 // Owner -> non-owner copy refresh (src/structured_halo.hpp:197 fused_halo_broadcast).
 // ---------------------------------------------------------------------------
@@ -209,128 +159,119 @@ __global__ void broadcast2_kernel(double2* __restrict__ X, const int32_t* __rest
     }
 }
 
-// ---------------------------------------------------------------------------
-// Fused structured-interior sweep.  One CTA = one tile of (CI-1) x (CJ-1)
-// DOFs; CI*CJ threads.  Phase 1 stages the (CI+1) x (CJ+1) node window in
-// shared memory; phase 2 evaluates each of the CI*CJ cells' four corner
-// samples ONCE (value, det, gradient and the role-contracted Hessian for the
-// three nodes each sample moves) - the reference re-evaluates every sample
-// for each of the 4 DOFs that share it; phase 3 gathers the 16-occurrence
-// patch of each DOF from its 4 cells, takes the 2x2 Newton step, backtracks
-// (<= 10 halvings) on the patch energy with the node substituted, applies
-// the omega blend and writes X_out.  Patch semantics follow
-// src/structured_patch.hpp:89-258 and src/sweep.hpp:1534-1650.
-// ---------------------------------------------------------------------------
-// Whether the fp32 line search reads T from phase 2's cell edges.  Measured
-// on B200: faster for shape (+1-2%) and untangle; shape_size runs 4-5%
-// slower with it (its line search keeps more values live, and the hoisted
-// edge loads spill), so it forms T from the staged positions instead.
-template <int KIND, class C> constexpr bool kEdgeCache2 = std::is_same_v<C, float> && KIND != kShapeSize;
-
-template <int CI, int CJ, class C, int KIND> struct TileShared2 {
-    static constexpr int NC = CI * CJ;
-    // fp32 cell edges for the mixed line search (one slot otherwise)
-    static constexpr int NE = kEdgeCache2<KIND, C> ? NC : 1;
-    // sample values: only the fp64 accept test reads them (one slot otherwise)
-    static constexpr int NM = std::is_same_v<C, double> ? NC : 1;
-    double2 P[(CI + 1) * (CJ + 1)];
-    C mu[4][NM];
-    C det[4][NC];
-    C gh[4][5][NC];  // per local corner a: gx, gy, hxx, hxy, hyy
-    float2 E[4][NE];  // axis-0 edge at column side 0, 1; axis-1 edge at row side 0, 1
-    uint8_t bad[NC]; // cell holds an inverted or badly shaped sample
-};
-
 // Mixed precision: a DOF whose patch touches a cell with an inverted sample or
 // a corner angle below asin(kBadCell) is relaxed entirely in fp64 (patch,
 // Newton step and line search), since accept/reject decisions next to such
 // cells are ill-conditioned in fp32.
 constexpr double kBadCell = 0.1;
 
-// Complete fp64 update of the DOF at window node (ti+1, tj+1): 16-occurrence
-// patch (W_inv = I) evaluated from the staged positions, 2x2 Newton step,
-// <= 10 halvings, omega blend.  Same semantics as the shared-sample path.
+// Complete fp64 update (or, grad_only, gradient) of one DOF by 16 lanes, one
+// per sample of its 2 x 2 cells (mask: those lanes, l this lane's sample):
+// P points to the upper left of its 3 x 3 nodes, PW the row length.  Every
+// lane returns the same point.  W_inv = I; 2x2 Newton step, <= 10 halvings,
+// omega blend.
+//
+// The accept test compares the energies of the 12 samples the DOF moves; the
+// four others add the same constant to both sides, and one of them that is
+// inverted (outside untangle) or has no finite metric rules every step out.  A
+// trial with a det <= 0 is refused (outside untangle) before its energies.
+//
+// One lane alone took some 5000 instructions for such a DOF (16 full samples
+// in fp64, and ten trials of 16 where an inverted sample keeps it in place)
+// while the rest of its warp waited: on a +-0.3 h grid, where 1% of the DOFs
+// touch a bad cell, that was a third of the sweep (2049^2: 280 us a sweep
+// against 208 at +-0.2 h; with 16 lanes 228).
 template <int KIND>
-__device__ double2 dof_update_fp64(const double2* __restrict__ P, int PW, int ti, int tj, double tx, double ty,
-                                   double delta, double omega, double2* gout = nullptr)
+__device__ __noinline__ double2 dof_fp64_lanes(const double2* __restrict__ P, int PW, int l, unsigned mask, double tx,
+                                               double ty, double delta, double omega, bool grad_only)
 {
-    const double2 pos = P[(ti + 1) * PW + (tj + 1)];
-    double g0 = 0, g1 = 0, hxx = 0, hxy = 0, hyy = 0, e0 = 0;
-    auto node = [&](int u, int v) { return P[(ti + u) * PW + (tj + v)]; };
-#pragma unroll 1
-    for (int cell = 0; cell < 4; ++cell) {
-        const int ci = cell >> 1, cj = cell & 1;
-        const int a = (1 - ci) * 2 + (1 - cj);
-#pragma unroll 1
-        for (int b = 0; b < 4; ++b) {
-            const double s0 = (b & 2) ? -1.0 : 1.0, s1 = (b & 1) ? -1.0 : 1.0;
-            const double2 pc = node(ci + (b >> 1), cj + (b & 1));
-            const int b0 = b ^ 2, b1 = b ^ 1;
-            const double2 p0 = node(ci + (b0 >> 1), cj + (b0 & 1));
-            const double2 p1 = node(ci + (b1 >> 1), cj + (b1 & 1));
-            SampleOut<double> o;
-            sample_full_c<KIND, double>(s0 * (p0.x - pc.x), s1 * (p1.x - pc.x), s0 * (p0.y - pc.y),
-                                        s1 * (p1.y - pc.y), delta, o);
-            e0 += o.mu;
-            if (b == a) {
-                g0 -= s0 * o.g[0] + s1 * o.g[1];
-                g1 -= s0 * o.g[2] + s1 * o.g[3];
-                hxx += o.H[0] + o.H[5] + s0 * s1 * (o.H[1] + o.H[4]);
-                hxy += o.H[2] + o.H[7] + s0 * s1 * (o.H[3] + o.H[6]);
-                hyy += o.H[10] + o.H[15] + s0 * s1 * (o.H[11] + o.H[14]);
-            } else if (b0 == a) {
-                g0 += s0 * o.g[0];
-                g1 += s0 * o.g[2];
-                hxx += o.H[0];
-                hxy += o.H[2];
-                hyy += o.H[10];
-            } else if (b1 == a) {
-                g0 += s1 * o.g[1];
-                g1 += s1 * o.g[3];
-                hxx += o.H[5];
-                hxy += o.H[7];
-                hyy += o.H[15];
-            }
-        }
+    const int ci = l >> 3, cj = (l >> 2) & 1, b = l & 3;
+    const int a = (1 - ci) * 2 + (1 - cj);
+    auto node = [&](int c) { return P[(ci + (c >> 1)) * PW + cj + (c & 1)]; };
+    auto sum = [&](double v) {
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) { v += __shfl_xor_sync(mask, v, o, 16); }
+        return v;
+    };
+    const double s0 = (b & 2) ? -1.0 : 1.0, s1 = (b & 1) ? -1.0 : 1.0;
+    const int role = b == a ? 0 : ((b ^ 2) == a ? 1 : ((b ^ 1) == a ? 2 : -1));
+    const double2 pc = node(b), p0 = node(b ^ 2), p1 = node(b ^ 1), pos = P[PW + 1];
+    const double ax = s0 * (p0.x - pc.x), bx = s1 * (p1.x - pc.x), ay = s0 * (p0.y - pc.y), by = s1 * (p1.y - pc.y);
+    SampleOut<double> o;
+    sample_full_c<KIND, double>(ax, bx, ay, by, delta, o);
+    double g0 = 0.0, g1 = 0.0, hxx = 0.0, hxy = 0.0, hyy = 0.0;
+    if (role == 0) {
+        g0 = -(s0 * o.g[0] + s1 * o.g[1]);
+        g1 = -(s0 * o.g[2] + s1 * o.g[3]);
+        hxx = o.H[0] + o.H[5] + s0 * s1 * (o.H[1] + o.H[4]);
+        hxy = o.H[2] + o.H[7] + s0 * s1 * (o.H[3] + o.H[6]);
+        hyy = o.H[10] + o.H[15] + s0 * s1 * (o.H[11] + o.H[14]);
+    } else if (role == 1) {
+        g0 = s0 * o.g[0];
+        g1 = s0 * o.g[2];
+        hxx = o.H[0];
+        hxy = o.H[2];
+        hyy = o.H[10];
+    } else if (role == 2) {
+        g0 = s1 * o.g[1];
+        g1 = s1 * o.g[3];
+        hxx = o.H[5];
+        hxy = o.H[7];
+        hyy = o.H[15];
     }
-    const double gv[2] = {g0 - tx, g1 - ty};
-    if (gout != nullptr) {
-        *gout = make_double2(gv[0], gv[1]);
-        return pos;
-    }
+    const double gv[2] = {sum(g0) - tx, sum(g1) - ty};
+    if (grad_only) { return make_double2(gv[0], gv[1]); }
+    hxx = sum(hxx);
+    hxy = sum(hxy);
+    hyy = sum(hyy);
+    const double e0 = sum(role >= 0 ? o.mu : 0.0);
+    if (__any_sync(mask, role < 0 && (!isfinite(o.mu) || (KIND != kUntangle && !(o.det > 0.0))))) { return pos; }
     const double Hm[4] = {hxx, hxy, hxy, hyy};
     double dl[2];
     solve2<double>(Hm, gv, dl);
+    // this lane's columns move by k0 d and k1 d
+    const double k0 = role == 0 ? -s0 : (role == 1 ? s0 : 0.0), k1 = role == 0 ? -s1 : (role == 2 ? s1 : 0.0);
     double alpha = 1.0;
 #pragma unroll 1
-    for (int it = 0; it < 10; ++it) {
+    for (int it = 0; it < 10; ++it, alpha *= 0.5) {
         const double dx = alpha * dl[0], dy = alpha * dl[1];
-        const double2 tr = make_double2(pos.x + dx, pos.y + dy);
-        double e = 0.0, md = INFINITY;
-#pragma unroll 1
-        for (int cell = 0; cell < 4; ++cell) {
-            const int ci = cell >> 1, cj = cell & 1;
-            const int a = (1 - ci) * 2 + (1 - cj);
-#pragma unroll 1
-            for (int b = 0; b < 4; ++b) {
-                const double s0 = (b & 2) ? -1.0 : 1.0, s1 = (b & 1) ? -1.0 : 1.0;
-                const int b0 = b ^ 2, b1 = b ^ 1;
-                const double2 pc = (b == a) ? tr : node(ci + (b >> 1), cj + (b & 1));
-                const double2 p0 = (b0 == a) ? tr : node(ci + (b0 >> 1), cj + (b0 & 1));
-                const double2 p1 = (b1 == a) ? tr : node(ci + (b1 >> 1), cj + (b1 & 1));
-                double d;
-                e += sample_mu_c<KIND, double>(s0 * (p0.x - pc.x), s1 * (p1.x - pc.x), s0 * (p0.y - pc.y),
-                                               s1 * (p1.y - pc.y), delta, d);
-                md = fmin(md, d);
-            }
-        }
-        e -= tx * dx + ty * dy;
-        if (isfinite(e) && e <= e0 + Tol<double>::energy && (KIND == kUntangle || md > 0.0)) {
+        const double t[4] = {ax + k0 * dx, bx + k1 * dx, ay + k0 * dy, by + k1 * dy};
+        if (KIND != kUntangle && __any_sync(mask, role >= 0 && !(det2(t) > 0.0))) { continue; }
+        const double e = sum(role >= 0 ? mu_value<double>(KIND, t, delta) : 0.0) - (tx * dx + ty * dy);
+        if (isfinite(e) && e <= e0 + Tol<double>::energy) {
             return make_double2(pos.x + omega * dx, pos.y + omega * dy);
         }
-        alpha *= 0.5;
     }
     return pos;
+}
+
+// The DOFs of a warp that need fp64 (`bad` on their lanes), two at a time by
+// dof_fp64_lanes; each lane passes its own DOF's window, slot and tau.  All 32
+// lanes call this.
+template <int KIND>
+__device__ __forceinline__ void warp_dofs_fp64(bool bad, const double2* P, int PW, int64_t slot, double2 tau,
+                                               double delta, double omega, double2* __restrict__ Xout,
+                                               double2* __restrict__ grad_out)
+{
+    unsigned todo = __ballot_sync(0xffffffffu, bad);
+    const int half = (threadIdx.x >> 4) & 1;
+    while (todo != 0u) {
+        const int first = __ffs(int(todo)) - 1;
+        todo &= todo - 1u;
+        const int second = todo != 0u ? __ffs(int(todo)) - 1 : -1;
+        todo &= todo - 1u;  // 0 stays 0
+        const int src = half == 0 ? first : (second >= 0 ? second : first);
+        const double2* Ps = reinterpret_cast<const double2*>(
+          __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(P), src));
+        const int64_t sl = __shfl_sync(0xffffffffu, slot, src);
+        const double tx = __shfl_sync(0xffffffffu, tau.x, src), ty = __shfl_sync(0xffffffffu, tau.y, src);
+        if (half == 0 || second >= 0) {
+            const double2 r = dof_fp64_lanes<KIND>(Ps, PW, threadIdx.x & 15, half ? 0xffff0000u : 0x0000ffffu, tx, ty,
+                                                   delta, omega, grad_out != nullptr);
+            if ((threadIdx.x & 15) == 0) { (grad_out != nullptr ? grad_out : Xout)[sl] = r; }
+        }
+        __syncwarp();
+    }
 }
 
 // fp64 metric change of one near-degenerate trial sample, from the staged
@@ -361,353 +302,234 @@ __device__ float dmu2_guard64(double2 qc, double2 q0, double2 q1, int role, doub
     return float(m1 - m0);
 }
 
-template <int CI, int CJ, int MINB, int KIND, class C, int FD>
-__global__ void __launch_bounds__(CI* CJ, MINB)
-  interior_tile_kernel(const double2* __restrict__ Xin, double2* __restrict__ Xout,
-                       const Tile2* __restrict__ tiles, const BlockInfo* __restrict__ blocks,
-                       const uint8_t* __restrict__ active, const double2* __restrict__ tau,
-                       double delta, double omega, double2* __restrict__ grad_out)
+// ---------------------------------------------------------------------------
+// Fused structured-interior sweep, fp64.  One CTA = one tile of CI x CJ DOFs,
+// one per thread, over the (CI+1) x (CJ+1) cells around them.  Phase 1 stages
+// the (CI+2) x (CJ+2) node window in shared memory; phase 2 evaluates each
+// cell's four corner samples ONCE (the reference re-evaluates every sample for
+// each of the 4 DOFs that share it) and stores the sums per cell corner:
+// gradient, contracted Hessian, and the energy of the three samples that move
+// that corner; phase 3 adds a DOF's four corners, takes the 2x2 Newton step,
+// backtracks (<= 10 halvings) on the energy of the 12 samples it moves, applies
+// the omega blend and writes X_out.  The four other samples of its patch add
+// the same constant to both sides of the accept test; one that is inverted
+// (outside untangle) or has no finite metric rules every step out (a bit per
+// sample and cell).  Patch semantics follow src/structured_patch.hpp:89-258
+// and src/sweep.hpp:1534-1650.
+//
+// fp64 issue bounds it (2049^2, +-0.3 h: 309 us a sweep; 365 before, 72 against
+// 95 at 1025^2).  The line search works on the 12 edges around the DOF
+// (only the four that meet there move) and divides once for two samples; after
+// a refused trial it looks at the dets first, so that a DOF held in place by an
+// inverted sample does not run ten full trials beside its warp.
+// The gradient and Hessian keep their order of operations: next to an almost
+// degenerate sample H holds (1/sine)^2 against 1, and a last bit there grows
+// by an order a sweep (a form with fewer operations ran 294 us, and moved such
+// nodes by 1e-1 h within ten sweeps).
+// NT > CI CJ: one round of phase 2 for every cell (small levels, where one
+// CTA's chain is the sweep's time).
+// ---------------------------------------------------------------------------
+template <int CI, int CJ> struct TileShared64 {
+    static constexpr int CH = CI + 1, CW = CJ + 1, NC = CH * CW;
+    double2 P[(CH + 1) * (CW + 1)];
+    double gh[4][6][NC];  // per cell corner: gx, gy, hxx, hxy, hyy, energy
+    uint8_t stop[NC];     // bit b: sample b rules out steps of the DOF it does not move
+};
+
+// Energies of two samples from their squared lengths and dets: s/(2D) each, on
+// one division (shape, untangle with the surrogate dets).
+template <int KIND>
+__device__ __forceinline__ double pair_energy64(double sa, double Da, double sb, double Db, double delta)
+{
+    if constexpr (KIND == kShapeSize) {
+        const double ma = sa / (2.0 * Da), mb = sb / (2.0 * Db), da = Da - 1.0, db = Db - 1.0;
+        return (ma * ma - 1.0 + da * da) + (mb * mb - 1.0 + db * db);
+    } else {
+        if constexpr (KIND == kUntangle) {
+            Da = untangle_dh(Da, delta);
+            Db = untangle_dh(Db, delta);
+        }
+        return (sa * Db + sb * Da) / (2.0 * (Da * Db)) - 2.0;
+    }
+}
+
+template <int CI, int CJ, int NT, int MINB, int KIND>
+__global__ void __launch_bounds__(NT, MINB)
+  interior_fp64_kernel(const double2* __restrict__ Xin, double2* __restrict__ Xout, const Tile2* __restrict__ tiles,
+                       const uint8_t* __restrict__ active, const double2* __restrict__ tau, double delta, double omega,
+                       double2* __restrict__ grad_out)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    // FD = 0: CI x CJ cells per CTA, one per thread, for their (CI-1) x (CJ-1)
-    // interior DOFs.  FD = 1: CI x CJ DOFs per CTA, one per thread, over the
-    // (CI+1) x (CJ+1) cells around them, so no thread idles in phase 3.
-    constexpr int NT = CI * CJ;
-    constexpr int CH = FD ? CI + 1 : CI, CW = FD ? CJ + 1 : CJ;  // cells staged
-    using S = TileShared2<CH, CW, C, KIND>;
+    using S = TileShared64<CI, CJ>;
     S& sm = *reinterpret_cast<S*>(smem_raw);
-    constexpr int NC = CH * CW;
-    constexpr int PW = CW + 1;
-
+    constexpr int NC = S::NC, CW = S::CW, PW = CW + 1;
     const Tile2 tile = tiles[blockIdx.x];
-    const BlockInfo bi = blocks[tile.block];
-    const int n0 = bi.n[0], n1 = bi.n[1];
+    const int n0 = tile.n0, n1 = tile.n1;
     const int r0 = tile.i0 - 1, c0 = tile.j0 - 1;  // node window origin
     const int tid = threadIdx.x;
 
     // Phase 1: node window.
-    for (int k = tid; k < (CH + 1) * PW; k += NT) {
+    for (int k = tid; k < (S::CH + 1) * PW; k += NT) {
         const int r = k / PW, c = k % PW;
         const int gi = r0 + r, gj = c0 + c;
         double2 v = make_double2(0.0, 0.0);
-        if (gi < n0 && gj < n1) { v = Xin[bi.off + int64_t(gi) * n1 + gj]; }
+        if (gi < n0 && gj < n1) { v = Xin[tile.off + int64_t(gi) * n1 + gj]; }
         sm.P[k] = v;
     }
+    // this thread's DOF, its flag and tau: in flight while phase 2 runs
+    const int ti = tid / CJ, tj = tid % CJ;
+    const int gi = tile.i0 + ti, gj = tile.j0 + tj;
+    const int64_t slot = tile.off + int64_t(gi) * n1 + gj;
+    const bool mine = tid < CI * CJ && gi <= n0 - 2 && gj <= n1 - 2 && active[slot];
+    double2 tv = make_double2(0.0, 0.0);
+    if (mine && tau != nullptr) { tv = tau[slot]; }
     __syncthreads();
 
-    // Phase 2: cell (ci, cj) with base node window (ci, cj); thread = cell
-    // (a second round for the extra cells of an FD tile).  Each thread
-    // accumulates the role contributions of its cell's four samples per
-    // corner in registers and stores them once to column `cell` of the shared
-    // cell arrays.
+    // Phase 2: cell (ci, cj) has its base at window node (ci, cj).
     for (int cell = tid; cell < NC; cell += NT) {
         const int ci = cell / CW, cj = cell % CW;
-        const bool valid = (r0 + ci <= n0 - 2) && (c0 + cj <= n1 - 2);
-        bool bad = false;
-        C acc[4][5];  // role contributions per cell corner, stored once below
+        if (r0 + ci > n0 - 2 || c0 + cj > n1 - 2) { continue; }  // read by no DOF
+        double acc[4][5], em[4];  // role contributions and moved energies per cell corner
+        unsigned stop = 0u;
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
 #pragma unroll
-            for (int q = 0; q < 5; ++q) { acc[a][q] = C(0); }
-            if constexpr (std::is_same_v<C, double>) { sm.mu[a][cell] = C(0); }
-            sm.det[a][cell] = C(1);
+            for (int q = 0; q < 5; ++q) { acc[a][q] = 0.0; }
+            em[a] = 0.0;
         }
-        if (valid) {
-            // The cell's four edges.  Sample b's columns are the axis-0 edge on
-            // side (b & 1) and the axis-1 edge on side (b >> 1): the sample
-            // signs cancel the edge orientation exactly, so T is bitwise the
-            // per-sample s_k (n_k - c).
-            const double2 p00 = sm.P[ci * PW + cj], p01 = sm.P[ci * PW + cj + 1];
-            const double2 p10 = sm.P[(ci + 1) * PW + cj], p11 = sm.P[(ci + 1) * PW + cj + 1];
-            const double e0x[2] = {p10.x - p00.x, p11.x - p01.x}, e0y[2] = {p10.y - p00.y, p11.y - p01.y};
-            const double e1x[2] = {p01.x - p00.x, p11.x - p10.x}, e1y[2] = {p01.y - p00.y, p11.y - p10.y};
-            if constexpr (kEdgeCache2<KIND, C>) {
+        // Sample b's columns are the axis-0 edge on side (b & 1) and the axis-1
+        // edge on side (b >> 1): the sample signs cancel the edge orientation.
+        const double2 p00 = sm.P[ci * PW + cj], p01 = sm.P[ci * PW + cj + 1];
+        const double2 p10 = sm.P[(ci + 1) * PW + cj], p11 = sm.P[(ci + 1) * PW + cj + 1];
+        const double e0x[2] = {p10.x - p00.x, p11.x - p01.x}, e0y[2] = {p10.y - p00.y, p11.y - p01.y};
+        const double e1x[2] = {p01.x - p00.x, p11.x - p10.x}, e1y[2] = {p01.y - p00.y, p11.y - p10.y};
 #pragma unroll
-                for (int k = 0; k < 2; ++k) {
-                    sm.E[k][cell] = make_float2(float(e0x[k]), float(e0y[k]));
-                    sm.E[2 + k][cell] = make_float2(float(e1x[k]), float(e1y[k]));
-                }
+        for (int b = 0; b < 4; ++b) {
+            const double s0 = (b & 2) ? -1.0 : 1.0;
+            const double s1 = (b & 1) ? -1.0 : 1.0;
+            RoleOut<double> o;
+            sample_roles_c<KIND, double>(e0x[b & 1], e1x[b >> 1], e0y[b & 1], e1y[b >> 1], s0, s1, delta, o);
+            if (!isfinite(o.mu) || (KIND != kUntangle && !(o.det > 0.0))) { stop |= 1u << b; }
+#pragma unroll
+            for (int q = 0; q < 5; ++q) {
+                acc[b][q] += o.r[0][q];
+                acc[b ^ 2][q] += o.r[1][q];
+                acc[b ^ 1][q] += o.r[2][q];
             }
-#pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                const double s0 = (b & 2) ? -1.0 : 1.0;
-                const double s1 = (b & 1) ? -1.0 : 1.0;
-                const double ax = e0x[b & 1], bx = e1x[b >> 1];
-                const double ay = e0y[b & 1], by = e1y[b >> 1];
-                if constexpr (std::is_same_v<C, float>) {
-                    // the fp32 / fp64 split needs only a coarse shape test
-                    const float fax = float(ax), fbx = float(bx), fay = float(ay), fby = float(by);
-                    const float dd = fax * fby - fbx * fay;
-                    const float nn = (fax * fax + fay * fay) * (fbx * fbx + fby * fby);
-                    bad = bad || !(dd > 0.0f) || dd * dd < float(kBadCell * kBadCell) * nn;
-                }
-                RoleOut<C> o;
-                sample_roles<KIND, C>(ax, bx, ay, by, s0, s1, delta, o);
-                if constexpr (std::is_same_v<C, double>) { sm.mu[b][cell] = o.mu; }  // fp32 accepts on differences
-                sm.det[b][cell] = o.det;
-#pragma unroll
-                for (int q = 0; q < 5; ++q) {
-                    acc[b][q] += o.r[0][q];
-                    acc[b ^ 2][q] += o.r[1][q];
-                    acc[b ^ 1][q] += o.r[2][q];
-                }
-            }
+            em[b] += o.mu;
+            em[b ^ 2] += o.mu;
+            em[b ^ 1] += o.mu;
         }
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
 #pragma unroll
             for (int q = 0; q < 5; ++q) { sm.gh[a][q][cell] = acc[a][q]; }
+            sm.gh[a][5][cell] = em[a];
         }
-        sm.bad[cell] = bad ? 1 : 0;
+        sm.stop[cell] = uint8_t(stop);
     }
     __syncthreads();
 
     // Phase 3: DOFs.
-    constexpr int DI = FD ? CI : CI - 1, DJ = FD ? CJ : CJ - 1;
-    if (tid >= DI * DJ) { return; }
-    const int ti = tid / DJ, tj = tid % DJ;
-    const int gi = tile.i0 + ti, gj = tile.j0 + tj;
-    if (gi > n0 - 2 || gj > n1 - 2) { return; }
-    const int64_t slot = bi.off + int64_t(gi) * n1 + gj;
-    if (!active[slot]) { return; }
-
-    C g0 = 0, g1 = 0, hxx = 0, hxy = 0, hyy = 0, e0 = 0, econst = 0;
-    C mdconst = C(INFINITY);
+    if (!mine) { return; }
+    const int c00 = ti * CW + tj;
+    double sum[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    unsigned stop = 0u;
 #pragma unroll
     for (int ci = 0; ci < 2; ++ci) {
 #pragma unroll
         for (int cj = 0; cj < 2; ++cj) {
-            const int cell = (ti + ci) * CW + (tj + cj);
-            const int a = (1 - ci) * 2 + (1 - cj);
-            g0 += sm.gh[a][0][cell];
-            g1 += sm.gh[a][1][cell];
-            hxx += sm.gh[a][2][cell];
-            hxy += sm.gh[a][3][cell];
-            hyy += sm.gh[a][4][cell];
-            if constexpr (std::is_same_v<C, double>) {  // energies: the fp64 accept test only
-                e0 += (sm.mu[0][cell] + sm.mu[1][cell]) + (sm.mu[2][cell] + sm.mu[3][cell]);
-                econst += sm.mu[a ^ 3][cell];
-            }
-            mdconst = fmin(mdconst, sm.det[a ^ 3][cell]);
+            const int cell = c00 + ci * CW + cj, a = (1 - ci) * 2 + (1 - cj);
+#pragma unroll
+            for (int q = 0; q < 6; ++q) { sum[q] += sm.gh[a][q][cell]; }
+            stop |= sm.stop[cell] & (1u << (a ^ 3));
         }
     }
-    C tx = 0, ty = 0;
-    double txd = 0.0, tyd = 0.0;
-    if (tau != nullptr) {
-        const double2 tv = tau[slot];
-        txd = tv.x;
-        tyd = tv.y;
-        tx = C(tv.x);
-        ty = C(tv.y);
-    }
-    if constexpr (std::is_same_v<C, float>) {
-        const int c00 = ti * CW + tj;
-        if (sm.bad[c00] | sm.bad[c00 + 1] | sm.bad[c00 + CW] | sm.bad[c00 + CW + 1]) {
-            if (grad_out != nullptr) {
-                dof_update_fp64<KIND>(sm.P, PW, ti, tj, txd, tyd, delta, omega, grad_out + slot);
-            } else {
-                Xout[slot] = dof_update_fp64<KIND>(sm.P, PW, ti, tj, txd, tyd, delta, omega);
-            }
-            return;
-        }
-    }
-    const C gv[2] = {g0 - tx, g1 - ty};
+    const double gv[2] = {sum[0] - tv.x, sum[1] - tv.y};
     if (grad_out != nullptr) {  // gradient-only mode (FAS restriction / tau)
-        grad_out[slot] = make_double2(double(gv[0]), double(gv[1]));
+        grad_out[slot] = make_double2(gv[0], gv[1]);
         return;
     }
-    const C Hm[4] = {hxx, hxy, hxy, hyy};
-    C dlt[2];
-    solve2<C>(Hm, gv, dlt);
+    double2 out = sm.P[(ti + 1) * PW + tj + 1];
+    if (stop != 0u) {
+        Xout[slot] = out;
+        return;
+    }
+    const double Hm[4] = {sum[2], sum[3], sum[3], sum[4]};
+    double dl[2];
+    solve2<double>(Hm, gv, dl);
 
-    // Neighbour offsets relative to the DOF, in working precision.
-    const double2 pos = sm.P[(ti + 1) * PW + (tj + 1)];
-    C rx[3][3], ry[3][3];
+    // The 12 edges around the DOF: V[c][k] down column tj + k from window row
+    // ti + c, H[r][k] along row ti + r from column tj + k; V[.][1] and H[1][.]
+    // meet at the DOF.
+    double Vx[2][3], Vy[2][3], Hx[3][2], Hy[3][2];
+    {
+        double2 up[3], at[3];
 #pragma unroll
-    for (int u = 0; u < 3; ++u) {
+        for (int r = 0; r < 3; ++r) {
 #pragma unroll
-        for (int v = 0; v < 3; ++v) {
-            const double2 q = sm.P[(ti + u) * PW + (tj + v)];
-            rx[u][v] = C(q.x - pos.x);
-            ry[u][v] = C(q.y - pos.y);
+            for (int k = 0; k < 3; ++k) {
+                at[k] = sm.P[(ti + r) * PW + tj + k];
+                if (r) {
+                    Vx[r - 1][k] = at[k].x - up[k].x;
+                    Vy[r - 1][k] = at[k].y - up[k].y;
+                }
+                if (k) {
+                    Hx[r][k - 1] = at[k].x - at[k - 1].x;
+                    Hy[r][k - 1] = at[k].y - at[k - 1].y;
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 3; ++k) { up[k] = at[k]; }
         }
     }
-
-    C alpha = C(1);
-    C ax_acc = C(0), ay_acc = C(0);
-    bool accepted = false;
-    if constexpr (std::is_same_v<C, float>) {
-        // fp32: accept on the summed metric changes of the 12 samples the DOF
-        // moves (dmu2, free of the cancellation of e' - e0 where mu ~ 1), with
-        // the fp64 energy tolerance; near-degenerate trial samples are
-        // differenced in fp64.
-        for (int it = 0; it < 10 && !accepted; ++it) {
-            const float dx = alpha * dlt[0], dy = alpha * dlt[1];
-            float dsum = 0.0f;
-            float md = mdconst;
-            unsigned guard = 0u;
+    double alpha = 1.0;
+#pragma unroll 1
+    for (int it = 0; it < 10; ++it, alpha *= 0.5) {
+        const double dx = alpha * dl[0], dy = alpha * dl[1];
+        // the moved edges: the upper and west ones end at the DOF, the others
+        // start there
+        const double vx[2] = {Vx[0][1] + dx, Vx[1][1] - dx}, vy[2] = {Vy[0][1] + dy, Vy[1][1] - dy};
+        const double hx[2] = {Hx[1][0] + dx, Hx[1][1] - dx}, hy[2] = {Hy[1][0] + dy, Hy[1][1] - dy};
+        // sample (ci, cj, r): the corner itself (both moved edges), the
+        // axis-0 neighbour (moved column edge, row edge of the outer row), the
+        // axis-1 neighbour (moved row edge, outer column edge)
+        auto sample = [&](int ci, int cj, int r, double& ax, double& ay, double& bx, double& by) {
+            ax = r == 2 ? Vx[ci][2 * cj] : vx[ci];
+            ay = r == 2 ? Vy[ci][2 * cj] : vy[ci];
+            bx = r == 1 ? Hx[2 * ci][cj] : hx[cj];
+            by = r == 1 ? Hy[2 * ci][cj] : hy[cj];
+        };
+        if (KIND != kUntangle && it > 0) {
+            double md = INFINITY;
+#pragma unroll
+            for (int k = 0; k < 12; ++k) {
+                double ax, ay, bx, by;
+                sample(k / 6, (k / 3) & 1, k % 3, ax, ay, bx, by);
+                md = fmin(md, ax * by - bx * ay);
+            }
+            if (!(md > 0.0)) { continue; }
+        }
+        double e = 0.0, md = INFINITY;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {  // samples (0, cj, r) and (1, cj, r)
+            double s[2], D[2];
 #pragma unroll
             for (int ci = 0; ci < 2; ++ci) {
-#pragma unroll
-                for (int cj = 0; cj < 2; ++cj) {
-                    const int a = (1 - ci) * 2 + (1 - cj);
-                    const int cell = (ti + ci) * CW + (tj + cj);
-#pragma unroll
-                    for (int r = 0; r < 3; ++r) {
-                        const int b = (r == 0) ? a : ((r == 1) ? (a ^ 2) : (a ^ 1));
-                        const float s0 = (b & 2) ? -1.0f : 1.0f;
-                        const float s1 = (b & 1) ? -1.0f : 1.0f;
-                        float t[4];
-                        if constexpr (kEdgeCache2<KIND, C>) {
-                            // T of sample b: the cell's fp32 edges from phase 2
-                            // (each rounded once from its fp64 difference)
-                            const float2 ea = sm.E[b & 1][cell], eb = sm.E[2 + (b >> 1)][cell];
-                            t[0] = ea.x;
-                            t[1] = eb.x;
-                            t[2] = ea.y;
-                            t[3] = eb.y;
-                        } else {
-                            const int bn0 = b ^ 2, bn1 = b ^ 1;
-                            const int cu = ci + (b >> 1), cv = cj + (b & 1);
-                            const int u0 = ci + (bn0 >> 1), v0 = cj + (bn0 & 1);
-                            const int u1 = ci + (bn1 >> 1), v1 = cj + (bn1 & 1);
-                            t[0] = s0 * (rx[u0][v0] - rx[cu][cv]);
-                            t[1] = s1 * (rx[u1][v1] - rx[cu][cv]);
-                            t[2] = s0 * (ry[u0][v0] - ry[cu][cv]);
-                            t[3] = s1 * (ry[u1][v1] - ry[cu][cv]);
-                        }
-                        // r = 0 moves both columns of T; r = 1 (2) moves column
-                        // 0 (1) only, whose change forms skip the zero entries.
-                        float dn, dm, ax, bx, ay, by;
-                        if (r == 0) {
-                            const float dt[4] = {-s0 * dx, -s1 * dx, -s0 * dy, -s1 * dy};
-                            dm = dmu2<float>(KIND, t, dt, float(delta), dn);
-                            ax = t[0] + dt[0];
-                            bx = t[1] + dt[1];
-                            ay = t[2] + dt[2];
-                            by = t[3] + dt[3];
-                        } else if (r == 1) {
-                            const float ex = s0 * dx, ey = s0 * dy;
-                            dm = dmu2_col<float, 0>(KIND, t, ex, ey, float(delta), dn);
-                            ax = t[0] + ex;
-                            bx = t[1];
-                            ay = t[2] + ey;
-                            by = t[3];
-                        } else {
-                            const float ex = s1 * dx, ey = s1 * dy;
-                            dm = dmu2_col<float, 1>(KIND, t, ex, ey, float(delta), dn);
-                            ax = t[0];
-                            bx = t[1] + ex;
-                            ay = t[2];
-                            by = t[3] + ey;
-                        }
-                        if (dn * dn < float(kGuard * kGuard) * (ax * ax + ay * ay) * (bx * bx + by * by)) {
-                            guard |= 1u << (ci * 6 + cj * 3 + r);  // redone in fp64 below
-                        } else {
-                            dsum += dm;
-                            md = fminf(md, dn);
-                        }
-                    }
-                }
+                double ax, ay, bx, by;
+                sample(ci, k / 3, k % 3, ax, ay, bx, by);
+                s[ci] = (ax * ax + ay * ay) + (bx * bx + by * by);
+                D[ci] = ax * by - bx * ay;
+                md = fmin(md, D[ci]);
             }
-#pragma unroll 1
-            for (int k = 0; guard && k < 12; ++k) {
-                if (!((guard >> k) & 1u)) { continue; }
-                const int ci = k / 6, cj = (k / 3) % 2, r = k % 3;
-                const int a = (1 - ci) * 2 + (1 - cj);
-                const int b = (r == 0) ? a : ((r == 1) ? (a ^ 2) : (a ^ 1));
-                const int bn0 = b ^ 2, bn1 = b ^ 1;
-                float dn;
-                dsum += dmu2_guard64<KIND>(sm.P[(ti + ci + (b >> 1)) * PW + (tj + cj + (b & 1))],
-                                           sm.P[(ti + ci + (bn0 >> 1)) * PW + (tj + cj + (bn0 & 1))],
-                                           sm.P[(ti + ci + (bn1 >> 1)) * PW + (tj + cj + (bn1 & 1))], r, double(dx),
-                                           double(dy), (b & 2) ? -1.0 : 1.0, (b & 1) ? -1.0 : 1.0, delta, dn);
-                md = fminf(md, dn);
-            }
-            dsum -= tx * dx + ty * dy;
-            if (isfinite(dsum) && dsum <= float(Tol<double>::energy) && (KIND == kUntangle || md > 0.0f)) {
-                ax_acc = dx;
-                ay_acc = dy;
-                accepted = true;
-            } else {
-                alpha *= 0.5f;
-            }
+            e += pair_energy64<KIND>(s[0], D[0], s[1], D[1], delta);
         }
-    } else {
-    for (int it = 0; it < 10 && !accepted; ++it) {
-        const C dx = alpha * dlt[0], dy = alpha * dlt[1];
-        C e = econst;
-        C md = mdconst;
-#pragma unroll
-        for (int ci = 0; ci < 2; ++ci) {
-#pragma unroll
-            for (int cj = 0; cj < 2; ++cj) {
-                const int a = (1 - ci) * 2 + (1 - cj);
-#pragma unroll
-                for (int r = 0; r < 3; ++r) {
-                    const int b = (r == 0) ? a : ((r == 1) ? (a ^ 2) : (a ^ 1));
-                    const int bn0 = b ^ 2, bn1 = b ^ 1;
-                    // node window coords of corner / neighbours (cell base (ci, cj))
-                    const int cu = ci + (b >> 1), cv = cj + (b & 1);
-                    const int u0 = ci + (bn0 >> 1), v0 = cj + (bn0 & 1);
-                    const int u1 = ci + (bn1 >> 1), v1 = cj + (bn1 & 1);
-                    const C pcx = (b == a) ? dx : rx[cu][cv];
-                    const C pcy = (b == a) ? dy : ry[cu][cv];
-                    const C p0x = (bn0 == a) ? dx : rx[u0][v0];
-                    const C p0y = (bn0 == a) ? dy : ry[u0][v0];
-                    const C p1x = (bn1 == a) ? dx : rx[u1][v1];
-                    const C p1y = (bn1 == a) ? dy : ry[u1][v1];
-                    const C s0 = (b & 2) ? C(-1) : C(1);
-                    const C s1 = (b & 1) ? C(-1) : C(1);
-                    C ax = s0 * (p0x - pcx), bx = s1 * (p1x - pcx);
-                    C ay = s0 * (p0y - pcy), by = s1 * (p1y - pcy);
-                    C d;
-                    C m;
-                    if constexpr (std::is_same_v<C, float>) {
-                        const float dd = ax * by - bx * ay;
-                        const float nn0 = ax * ax + ay * ay, nn1 = bx * bx + by * by;
-                        if (dd * dd < float(kGuard * kGuard) * nn0 * nn1) {
-                            // fp64 re-evaluation from the staged fp64 positions
-                            const double2 qc = sm.P[(ti + cu) * PW + (tj + cv)];
-                            const double2 q0 = sm.P[(ti + u0) * PW + (tj + v0)];
-                            const double2 q1 = sm.P[(ti + u1) * PW + (tj + v1)];
-                            const double tX = pos.x + double(dx), tY = pos.y + double(dy);
-                            const double cX = (b == a) ? tX : qc.x, cY = (b == a) ? tY : qc.y;
-                            const double X0 = (bn0 == a) ? tX : q0.x, Y0 = (bn0 == a) ? tY : q0.y;
-                            const double X1 = (bn1 == a) ? tX : q1.x, Y1 = (bn1 == a) ? tY : q1.y;
-                            double dd64;
-                            const double m64 = sample_mu_c<KIND, double>(
-                              double(s0) * (X0 - cX), double(s1) * (X1 - cX), double(s0) * (Y0 - cY),
-                              double(s1) * (Y1 - cY), delta, dd64);
-                            m = float(m64);
-                            d = float(dd64);
-                        } else {
-                            m = sample_mu_c<KIND, float>(ax, bx, ay, by, float(delta), d);
-                        }
-                    } else {
-                        m = sample_mu_c<KIND, double>(ax, bx, ay, by, delta, d);
-                    }
-                    e += m;
-                    md = fmin(md, d);
-                }
-            }
+        e -= tv.x * dx + tv.y * dy;
+        if (isfinite(e) && e <= sum[5] + Tol<double>::energy && (KIND == kUntangle || md > 0.0)) {
+            out.x += omega * dx;
+            out.y += omega * dy;
+            break;
         }
-        e -= tx * dx + ty * dy;
-        const bool ok = isfinite(e) && (e <= e0 + Tol<C>::energy) &&
-                        (KIND == kUntangle || md > C(0));
-        if (ok) {
-            ax_acc = dx;
-            ay_acc = dy;
-            accepted = true;
-        } else {
-            alpha *= C(0.5);
-        }
-    }
-    }
-    double2 out = pos;
-    if (accepted) {
-        out.x = pos.x + omega * double(ax_acc);
-        out.y = pos.y + omega * double(ay_acc);
     }
     Xout[slot] = out;
 }

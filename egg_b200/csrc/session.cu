@@ -99,10 +99,13 @@ template <class T> struct DevBuf {
 // minimum resident CTAs per SM requested from the register allocator.  The
 // session's autotuner times each on the session's own data and keeps the
 // fastest (egg_b200_session_autotune).
-// 2D: (ci, cj) cells per CTA, or with fd = 1 (ci, cj) DOFs per CTA over the
-// (ci+1) x (cj+1) cells around them; fd = 2 is the same full-DOF tile on the
-// packed two-lane fp32 kernel (interior_x2_kernel, mixed precision only), fd
-// = 3 its persistent form with TMA window prefetch (interior_x2p_kernel);
+// 2D: (ci, cj) DOFs per CTA over the (ci+1) x (cj+1) cells around them; fp64
+// with one thread per DOF (fd = 1) or per cell (fd = 4); fd = 2 is the packed
+// two-lane fp32 kernel (interior_x2_kernel, mixed precision only).  us a sweep
+// of a 2049^2 / 1025^2 / 257^2 square (+-0.3 h, shape) in the tables' order:
+// fp64 309 / 72 / 10.6, 312 / 75 / 10.5, 315 / 76 / 10.6, 340 / 83 / 10.5;
+// mixed 201 / 50 / 8.5, 214 / 55 / 10, 208 / 53 / 8.5,
+// 226 / 58 / 8.5, 212 / 52 / 8.5.
 // 3D: (ci, cj, ck) DOFs per CTA.
 struct Variant {
     int ci, cj, ck, minb, fd = 0;
@@ -110,8 +113,8 @@ struct Variant {
 constexpr int kNumVariants = EGG_B200_NUM_VARIANTS;
 // Host threads that copy X between the caller's buffer and pinned staging.
 constexpr int kMaxCopyThreads = 16;
-constexpr Variant kVar64[kNumVariants] = {{8, 16, 1, 5, 1}, {8, 16, 1, 4}, {8, 16, 1, 5}, {8, 16, 1, 6}, {8, 16, 1, 4, 1}};
-constexpr Variant kVar32[kNumVariants] = {{8, 16, 1, 7, 2}, {8, 16, 1, 8, 2}, {8, 16, 1, 6, 2}, {8, 16, 1, 5, 2}, {8, 16, 1, 7, 3}};
+constexpr Variant kVar64[kNumVariants] = {{8, 16, 1, 4, 1}, {8, 16, 1, 4, 4}, {8, 16, 1, 5, 1}, {16, 16, 1, 2, 1}, {8, 16, 1, 3, 1}};
+constexpr Variant kVar32[kNumVariants] = {{8, 16, 1, 7, 2}, {8, 16, 1, 8, 2}, {8, 16, 1, 6, 2}, {8, 16, 1, 5, 2}, {4, 24, 1, 9, 2}};
 // 3D (interior3_kernel), us a sweep of a 129^3 / 59^3 / 33^3 cube, in the table's
 // order: fp64 969 / 125 / 25.0, 957 / 112 / 26.9, 963 / 120 / 27.0,
 // 1029 / 120 / 28.3, 975 / 125 / 27.2; mixed 545 / 72 / 16.8, 556 / 72 / 16.7,
@@ -188,10 +191,7 @@ struct Session : LevelData {
     int prec = EGG_B200_PREC_FP64;
     int device = 0;
     int num_sms = 148;
-    // error flag of kernels with bounded waits (set on device, checked at sync)
-    DevBuf<int> kerr;
-    bool kerr_armed = false;
-    cudaStream_t stream = nullptr;
+        cudaStream_t stream = nullptr;
     // side stream + fork/join events: the stored-patch sweep runs beside the
     // interior tiles (both read the frozen snapshot, write disjoint slots)
     cudaStream_t side = nullptr;
@@ -349,20 +349,6 @@ struct Session : LevelData {
     {
         EGG_CK(cudaStreamSynchronize(stream));
         harvest();
-        check_kerr();
-    }
-
-    // A kernel whose bounded wait ran out set kerr: report it once as an error.
-    void check_kerr()
-    {
-        if (!kerr_armed || kerr.p == nullptr) { return; }
-        kerr_armed = false;
-        int e = 0;
-        EGG_CK(cudaMemcpy(&e, kerr.p, sizeof(int), cudaMemcpyDeviceToHost));
-        if (e != 0) {
-            EGG_CK(cudaMemset(kerr.p, 0, sizeof(int)));
-            throw Error(EGG_B200_ERUNTIME, "interior sweep: a window copy did not complete within its wait limit");
-        }
     }
 
     double* X(int i) { return Xbuf[i].p; }
@@ -466,69 +452,58 @@ static bool rows_uniform(const double* W, int64_t rows, int width)
     return true;
 }
 
-// Opt the interior kernels into >48 KB of dynamic shared memory.
-template <int CI, int CJ, int FD, int KIND, class C> constexpr size_t tile_smem2()
+// Threads of the 2D fp64 tile kernel: one per DOF, or (fd = 4) one per cell in
+// whole warps.
+template <int CI, int CJ, int FD> constexpr int threads64() { return FD == 4 ? ((CI + 1) * (CJ + 1) + 31) / 32 * 32 : CI * CJ; }
+
+// Opt the 2D interior kernels into >48 KB of dynamic shared memory.
+template <int CI, int CJ, int FD, class C> constexpr size_t tile_smem2()
 {
     if constexpr (FD == 2) {
         return sizeof(TileSharedX2<CI, CJ>);
-    } else if constexpr (FD == 3) {
-        return sizeof(TileSharedX2<CI, CJ, 2>);
     } else {
-        return sizeof(TileShared2<CI + FD, CJ + FD, C, KIND>);
+        return sizeof(TileShared64<CI, CJ>);
     }
+}
+
+template <int CI, int CJ, int MINB, int FD, int KIND, class C> static void set_smem_attr_kind()
+{
+    constexpr int sz = int(tile_smem2<CI, CJ, FD, C>());
+    static_assert((FD == 2) == std::is_same_v<C, float>, "the packed kernel is the mixed-precision path");
+    const void* f = nullptr;
+    if constexpr (FD == 2) {
+        f = reinterpret_cast<const void*>(interior_x2_kernel<CI, CJ, MINB, KIND>);
+    } else {
+        f = reinterpret_cast<const void*>(interior_fp64_kernel<CI, CJ, threads64<CI, CJ, FD>(), MINB, KIND>);
+    }
+    EGG_CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, sz));
 }
 
 template <int CI, int CJ, int MINB, class C, int FD> static void set_smem_attr()
 {
-    if constexpr (FD == 3) {
-        static_assert(std::is_same_v<C, float>, "the packed kernel is the mixed-precision path");
-        constexpr int sz = int(sizeof(TileSharedX2<CI, CJ, 2>));
-        EGG_CK(cudaFuncSetAttribute(interior_x2p_kernel<CI, CJ, MINB, kShape>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, sz));
-        EGG_CK(cudaFuncSetAttribute(interior_x2p_kernel<CI, CJ, MINB, kUntangle>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, sz));
-        EGG_CK(cudaFuncSetAttribute(interior_x2p_kernel<CI, CJ, MINB, kShapeSize>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, sz));
-        return;
-    } else if constexpr (FD == 2) {
-        static_assert(std::is_same_v<C, float>, "the packed kernel is the mixed-precision path");
-        EGG_CK(cudaFuncSetAttribute(interior_x2_kernel<CI, CJ, MINB, kShape>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(TileSharedX2<CI, CJ>))));
-        EGG_CK(cudaFuncSetAttribute(interior_x2_kernel<CI, CJ, MINB, kUntangle>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(TileSharedX2<CI, CJ>))));
-        EGG_CK(cudaFuncSetAttribute(interior_x2_kernel<CI, CJ, MINB, kShapeSize>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(TileSharedX2<CI, CJ>))));
-        return;
-    } else {
-    EGG_CK(cudaFuncSetAttribute(interior_tile_kernel<CI, CJ, MINB, kShape, C, FD>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, int(tile_smem2<CI, CJ, FD, kShape, C>())));
-    EGG_CK(cudaFuncSetAttribute(interior_tile_kernel<CI, CJ, MINB, kUntangle, C, FD>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                int(tile_smem2<CI, CJ, FD, kUntangle, C>())));
-    EGG_CK(cudaFuncSetAttribute(interior_tile_kernel<CI, CJ, MINB, kShapeSize, C, FD>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                int(tile_smem2<CI, CJ, FD, kShapeSize, C>())));
-    }
+    set_smem_attr_kind<CI, CJ, MINB, FD, kShape, C>();
+    set_smem_attr_kind<CI, CJ, MINB, FD, kUntangle, C>();
+    set_smem_attr_kind<CI, CJ, MINB, FD, kShapeSize, C>();
 }
 
 static void configure_kernels(int prec, int dim)
 {
-    if (dim == 3) { return; }  // 3D kernels use < 48 KB of static shared memory
+    if (dim == 3) { return; }  // 3D kernels use < 48 KB of shared memory
+#define EGG_SMEM(T, C, i) set_smem_attr<T[i].ci, T[i].cj, T[i].minb, C, T[i].fd>()
+    EGG_SMEM(kVar64, double, 0);  // also the coarsest FAS level of a mixed session
     if (prec == EGG_B200_PREC_FP64) {
-        set_smem_attr<kVar64[0].ci, kVar64[0].cj, kVar64[0].minb, double, kVar64[0].fd>();
-        set_smem_attr<kVar64[1].ci, kVar64[1].cj, kVar64[1].minb, double, kVar64[1].fd>();
-        set_smem_attr<kVar64[2].ci, kVar64[2].cj, kVar64[2].minb, double, kVar64[2].fd>();
-        set_smem_attr<kVar64[3].ci, kVar64[3].cj, kVar64[3].minb, double, kVar64[3].fd>();
-        set_smem_attr<kVar64[4].ci, kVar64[4].cj, kVar64[4].minb, double, kVar64[4].fd>();
+        EGG_SMEM(kVar64, double, 1);
+        EGG_SMEM(kVar64, double, 2);
+        EGG_SMEM(kVar64, double, 3);
+        EGG_SMEM(kVar64, double, 4);
     } else {
-        set_smem_attr<kVar32[0].ci, kVar32[0].cj, kVar32[0].minb, float, kVar32[0].fd>();
-        set_smem_attr<kVar32[1].ci, kVar32[1].cj, kVar32[1].minb, float, kVar32[1].fd>();
-        set_smem_attr<kVar32[2].ci, kVar32[2].cj, kVar32[2].minb, float, kVar32[2].fd>();
-        set_smem_attr<kVar32[3].ci, kVar32[3].cj, kVar32[3].minb, float, kVar32[3].fd>();
-        set_smem_attr<kVar32[4].ci, kVar32[4].cj, kVar32[4].minb, float, kVar32[4].fd>();
-        // the coarsest FAS level of a mixed session runs the first fp64 variant
-        set_smem_attr<kVar64[0].ci, kVar64[0].cj, kVar64[0].minb, double, kVar64[0].fd>();
+        EGG_SMEM(kVar32, float, 0);
+        EGG_SMEM(kVar32, float, 1);
+        EGG_SMEM(kVar32, float, 2);
+        EGG_SMEM(kVar32, float, 3);
+        EGG_SMEM(kVar32, float, 4);
     }
+#undef EGG_SMEM
 }
 
 static Variant variant_shape(const Session& S, int v)
@@ -538,15 +513,13 @@ static Variant variant_shape(const Session& S, int v)
 }
 
 // Tile list of the interior kernel for variant v over every block's
-// structured interior, keeping tiles that hold a moving DOF.  2D: CI x CJ
-// cells, (CI-1) x (CJ-1) DOFs per tile (CI x CJ DOFs with fd); 3D: CI x CJ x
-// CK DOFs per tile.
+// structured interior, keeping tiles that hold a moving DOF: CI x CJ (x CK)
+// DOFs per tile.
 static void set_tiles(Session& S, LevelData& L, Variant v)
 {
     if (L.tile_ci == v.ci && L.tile_cj == v.cj && L.tile_ck == v.ck && L.tile_fd == v.fd) { return; }
     S.drop_graphs();
-    const int shrink = (S.dim == 2 && !v.fd) ? 1 : 0;
-    const int di = v.ci - shrink, dj = v.cj - shrink, dk = S.dim == 2 ? 1 : v.ck;
+    const int di = v.ci, dj = v.cj, dk = S.dim == 2 ? 1 : v.ck;
     std::vector<Tile2> tiles2;
     std::vector<Tile3> tiles3;
     for (int b = 0; b < int(L.blocks_h.size()); ++b) {
@@ -570,7 +543,7 @@ static void set_tiles(Session& S, LevelData& L, Variant v)
                     }
                     if (!any) { continue; }
                     if (S.dim == 2) {
-                        tiles2.push_back(Tile2 {b, i0, j0, 0});
+                        tiles2.push_back(Tile2 {bi.off, bi.n[0], bi.n[1], i0, j0, {0, 0}});
                     } else {
                         tiles3.push_back(Tile3 {b, i0, j0, k0});
                     }
@@ -1260,7 +1233,6 @@ static Session* create_session(const egg_b200_session_desc& d)
     EGG_CK(cudaEventCreateWithFlags(&S->join_ev, cudaEventDisableTiming));
     configure_kernels(S->prec, S->dim);
     EGG_CK(cudaDeviceGetAttribute(&S->num_sms, cudaDevAttrMultiProcessorCount, S->device));
-    S->kerr.upload(std::vector<int> {0});
 
     // ---- upload -----------------------------------------------------------
     S->es_W.upload(es_W_h);
@@ -1386,31 +1358,18 @@ template <int CI, int CJ, int MINB, int KIND, class C, int FD>
 static void launch_tile(Session& S, LevelData& L, const double* xin, double* xout, const double* tau, double delta,
                         double omega, double* gout)
 {
-    const size_t smem = tile_smem2<CI, CJ, FD, KIND, C>();
+    const size_t smem = tile_smem2<CI, CJ, FD, C>();
     const auto* xi = reinterpret_cast<const double2*>(xin);
     auto* xo = reinterpret_cast<double2*>(xout);
     const auto* tv = reinterpret_cast<const double2*>(tau);
     S.timed(kKInterior, [&] {
-        if constexpr (FD == 3) {
-            // persistent: as many CTAs as fit on the device at once
-            static const int per_sm = [] {
-                int nb = 0;
-                EGG_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                  &nb, interior_x2p_kernel<CI, CJ, MINB, KIND>, TileSharedX2<CI, CJ, 2>::NT,
-                  sizeof(TileSharedX2<CI, CJ, 2>)));
-                return std::max(nb, 1);
-            }();
-            const int grid = int(std::min<int64_t>(L.ntiles, int64_t(per_sm) * S.num_sms));
-            interior_x2p_kernel<CI, CJ, MINB, KIND><<<unsigned(grid), TileSharedX2<CI, CJ, 2>::NT, smem, S.stream>>>(
-              xi, xo, L.tiles_d.p, int(L.ntiles), L.blocks_d.p, L.active_d.p, tv, delta, omega,
-              reinterpret_cast<double2*>(gout), S.kerr.p);
-            S.kerr_armed = true;
-        } else if constexpr (FD == 2) {
+        if constexpr (FD == 2) {
             interior_x2_kernel<CI, CJ, MINB, KIND><<<unsigned(L.ntiles), TileSharedX2<CI, CJ>::NT, smem, S.stream>>>(
-              xi, xo, L.tiles_d.p, L.blocks_d.p, L.active_d.p, tv, delta, omega, reinterpret_cast<double2*>(gout));
+              xi, xo, L.tiles_d.p, L.active_d.p, tv, delta, omega, reinterpret_cast<double2*>(gout));
         } else {
-            interior_tile_kernel<CI, CJ, MINB, KIND, C, FD><<<unsigned(L.ntiles), CI * CJ, smem, S.stream>>>(
-              xi, xo, L.tiles_d.p, L.blocks_d.p, L.active_d.p, tv, delta, omega, reinterpret_cast<double2*>(gout));
+            constexpr int NT = threads64<CI, CJ, FD>();
+            interior_fp64_kernel<CI, CJ, NT, MINB, KIND><<<unsigned(L.ntiles), NT, smem, S.stream>>>(
+              xi, xo, L.tiles_d.p, L.active_d.p, tv, delta, omega, reinterpret_cast<double2*>(gout));
         }
     });
 }

@@ -68,7 +68,7 @@ X2_HD float2 fma2(float2 a, float2 b, float2 c)
 // correctly rounded difference.
 X2_HD float2 sub2(float2 a, float2 b) { return fma2(b, p2(-1.0f), a); }
 
-X2_HD float2 neg2(float2 a) { return mul2(a, p2(-1.0f)); }
+X2_HD float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
 
 // Per-lane quotient with the same division as the scalar fp32 line search.
 X2_HD float2 ldiv2(float2 a, float2 b) { return make_float2(ls_div(a.x, b.x), ls_div(a.y, b.y)); }
