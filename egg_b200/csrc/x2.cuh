@@ -82,11 +82,18 @@ template <int KIND> X2_HD Scale2 scale2(float2 s, float2 D, float delta)
 {
     Scale2 o;
     if constexpr (KIND == kUntangle) {
-        const ScaleFn<float> fx = untangle_scale(D.x, delta), fy = untangle_scale(D.y, delta);
-        o.twof = make_float2(2.0f * fx.f, 2.0f * fy.f);
-        o.A = make_float2(2.0f * fx.fp, 2.0f * fy.fp);
-        o.B = mul2(s, make_float2(fx.fpp, fy.fpp));
-        o.sfp = mul2(s, make_float2(fx.fp, fy.fp));
+        // untangle_scale with one quotient 1/r for Dh' = Dh / r and Dh'' =
+        // 2 delta^2 / r^3: 2f = 1/Dh, 2f' = -Dh'/Dh^2, 2f'' = -Dh''/Dh^2 + 2 Dh'^2/Dh^3
+        const float2 q = fma2(D, D, p2(4.0f * delta * delta));
+        const float2 r = make_float2(sqrtf(q.x), sqrtf(q.y));
+        const float2 Dh = mul2(p2(0.5f), add2(D, r));
+        const float2 ir = make_float2(1.0f / r.x, 1.0f / r.y), inv = make_float2(1.0f / Dh.x, 1.0f / Dh.y);
+        const float2 d1 = mul2(Dh, ir), d2 = mul2(mul2(p2(2.0f * delta * delta), ir), mul2(ir, ir));
+        const float2 inv2 = mul2(inv, inv), d1i = mul2(d1, inv);
+        o.twof = inv;
+        o.A = neg2(mul2(d1, inv2));
+        o.B = mul2(s, mul2(inv, fma2(d1i, d1i, mul2(p2(-0.5f), mul2(d2, inv)))));
+        o.sfp = mul2(mul2(s, p2(0.5f)), o.A);
     } else {
         // f = 1/(2D): 2f = 1/D, 2f' = -1/D^2, s f'' = s/D^3, s f' = -s/(2D^2)
         const float2 inv = make_float2(1.0f / D.x, 1.0f / D.y);
@@ -201,6 +208,19 @@ X2_HD float2 dmu2_pair(float2 s, float2 D, float2 twoD, float2 m2, float2 ds, fl
 {
     dn = add2(D, dD);
     if constexpr (KIND == kUntangle) {
+        // all four dets positive (all but the cells still tangled): the
+        // cancellation-free branch of untangle_dh_stable and untangle_ddh, in
+        // two lanes
+        if (fminf(fminf(D.x, D.y), fminf(dn.x, dn.y)) >= 0.0f) {
+            const float2 d2 = p2(4.0f * delta * delta);
+            const float2 q = fma2(D, D, d2), qn = fma2(dn, dn, d2);
+            const float2 r = make_float2(sqrtf(q.x), sqrtf(q.y)), rn = make_float2(sqrtf(qn.x), sqrtf(qn.y));
+            const float2 twoDh = add2(D, r), twoDhn = add2(dn, rn);
+            const float2 c = ldiv2(add2(dn, D), add2(rn, r));
+            const float2 twodDh = fma2(dD, c, dD);
+            // (ds Dh - s dDh) / (2 Dh Dh')
+            return ldiv2(fma2(ds, twoDh, neg2(mul2(s, twodDh))), mul2(twoDh, twoDhn));
+        }
         float ax, ay;
         const float rx = dmu2_from<float>(kUntangle, s.x, D.x, ds.x, dD.x, delta, ax);
         const float ry = dmu2_from<float>(kUntangle, s.y, D.y, ds.y, dD.y, delta, ay);
