@@ -539,6 +539,15 @@ __global__ void __launch_bounds__(NT, MINB)
 // slice; general W_inv, per-sample weights and the FAS tau shift.  Mirrors
 // src/patch.hpp:325 patch_eval + src/sweep.hpp:1534 interior_update_kernel.
 // ---------------------------------------------------------------------------
+// The non-owner copies of stored DOFs (slots dst[off[d] .. off[d + 1]) of DOF d,
+// off == NULL: none).  A relaxed node is written to its copies with it, so a
+// sweep needs no owner -> copy launch of its own (3 us of the 12 us sweep of a
+// 5 x 65^2 disk); a node that no DOF moves keeps the copies it started with.
+struct Copies {
+    const int32_t* off;
+    const int32_t* dst;
+};
+
 struct StoredPatch2 {
     int64_t n;              // DOFs
     const int32_t* slot;    // [n] owner slot of each DOF
@@ -559,6 +568,7 @@ struct StoredPatch2 {
     const double* arena;    // entity arena (B-spline knots, control points, weights)
     double* seeds;          // [n] last foot parameter of each B-spline DOF (NaN: none)
     SoftTable soft;         // directional / curvature terms per DOF (off == NULL: none)
+    Copies copies;
 };
 
 __device__ __forceinline__ void assemble_T(const double2 c, const double2 n0, const double2 n1,
@@ -839,7 +849,12 @@ __global__ void stored_patch_kernel(StoredPatch2 sp, const double2* __restrict__
             cur.y = pos.y + omega * (cur.y - pos.y);
         }
         if (bsp && lane == 0) { sp.seeds[d] = seed; }
-        if (lane == 0) { Xout[slot] = cur; }
+        if (lane == 0) {
+            Xout[slot] = cur;
+            if (sp.copies.off != nullptr) {
+                for (int32_t c = sp.copies.off[d]; c < sp.copies.off[d + 1]; ++c) { Xout[sp.copies.dst[c]] = cur; }
+            }
+        }
     }
 }
 

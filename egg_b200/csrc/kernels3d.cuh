@@ -426,6 +426,7 @@ struct StoredPatch3 {
     SoftTable soft;      // directional terms per DOF (off == NULL: none)
     const double* arena; // entity arena (B-spline surfaces)
     double* seeds;       // [n * 2] last foot parameter of each B-spline-surface DOF (NaN: none)
+    Copies copies;
 };
 
 __device__ __forceinline__ void assemble_T3(const double* X, int32_t ic, const int32_t in[3], const double s[3],
@@ -471,6 +472,7 @@ __device__ __forceinline__ void assemble_T3(const double* X, int32_t ic, const i
 struct Lattice3 {
     int64_t n;            // DOFs
     const int32_t* node;  // [27][n] node slots, entry 13 the DOF
+    Copies copies;
 };
 constexpr int kLatDofs = 64;  // DOFs per CTA of 2 kLatDofs threads
 struct WinLat3 {
@@ -514,6 +516,11 @@ __device__ __noinline__ void lattice3_cta(double* P, Lattice3 lat, int64_t d0, c
     double* dst = go ? grad_out : Xout;
 #pragma unroll
     for (int q = 0; q < 3; ++q) { dst[3 * slot + q] = out[q]; }
+    if (!go && lat.copies.off != nullptr) {
+        for (int32_t c = lat.copies.off[d]; c < lat.copies.off[d + 1]; ++c) {
+            for (int q = 0; q < 3; ++q) { Xout[3 * int64_t(lat.copies.dst[c]) + q] = out[q]; }
+        }
+    }
 }
 
 // Stored-patch sweep, 3D, G lanes per DOF (see stored_patch_kernel): the
@@ -667,7 +674,13 @@ __global__ void stored3_kernel(StoredPatch3 sp, int nb, Lattice3 lat, const doub
         }
         if (lane == 0) {
             for (int q = 0; q < 3; ++q) {
-                Xout[3 * int64_t(slot) + q] = etag != 0 ? cur[q] : pos[q] + omega * (cur[q] - pos[q]);
+                cur[q] = etag != 0 ? cur[q] : pos[q] + omega * (cur[q] - pos[q]);
+                Xout[3 * int64_t(slot) + q] = cur[q];
+            }
+            if (sp.copies.off != nullptr) {
+                for (int32_t c = sp.copies.off[d]; c < sp.copies.off[d + 1]; ++c) {
+                    for (int q = 0; q < 3; ++q) { Xout[3 * int64_t(sp.copies.dst[c]) + q] = cur[q]; }
+                }
             }
             if (bsurf) {
                 sp.seeds[2 * d] = seed[0];

@@ -161,6 +161,8 @@ struct LevelData {
     // not among the n_stored below
     int64_t n_lat = 0;
     DevBuf<int32_t> lat_node;
+    // the copies of the stored and the lattice DOFs (empty without shared nodes)
+    DevBuf<int32_t> st_cp_off, st_cp_dst, lat_cp_off, lat_cp_dst;
     int64_t n_stored = 0;
     DevBuf<int32_t> st_slot, st_gc, st_gn0, st_gn1, st_gn2, st_role;
     DevBuf<int64_t> st_off;
@@ -565,6 +567,39 @@ static void set_tiles(Session& S, LevelData& L, Variant v)
 }
 
 #include "lattice_host.inc"
+
+// Copies tables of a level's stored and lattice DOFs from its owner -> copy
+// pairs.
+static void upload_copies(LevelData& L, const std::vector<int32_t>& sh_src, const std::vector<int32_t>& sh_dst,
+                          const std::vector<int32_t>& st_slot, const std::vector<int32_t>& lat_node)
+{
+    if (sh_src.empty()) { return; }
+    const size_t ns = st_slot.size(), nl = lat_node.size() / 27;
+    std::vector<int32_t> of(size_t(L.nstore), -1), off(ns + nl + 1, 0);  // DOF of an owner slot
+    for (size_t d = 0; d < ns + nl; ++d) {
+        of[size_t(d < ns ? st_slot[d] : lat_node[13 * nl + (d - ns)])] = int32_t(d);
+    }
+    for (int32_t s : sh_src) {
+        if (of[size_t(s)] >= 0) { ++off[size_t(of[size_t(s)]) + 1]; }
+    }
+    for (size_t d = 0; d < ns + nl; ++d) { off[d + 1] += off[d]; }
+    std::vector<int32_t> at(off.begin(), off.end() - 1), dst(size_t(off.back()));
+    for (size_t e = 0; e < sh_src.size(); ++e) {
+        const int32_t d = of[size_t(sh_src[e])];
+        if (d >= 0) { dst[size_t(at[size_t(d)]++)] = sh_dst[e]; }
+    }
+    const size_t cut = size_t(off[ns]);
+    std::vector<int32_t> lat_off(off.begin() + std::ptrdiff_t(ns), off.end());
+    for (int32_t& v : lat_off) { v -= int32_t(cut); }
+    if (cut) {
+        L.st_cp_off.upload(std::vector<int32_t>(off.begin(), off.begin() + std::ptrdiff_t(ns) + 1));
+        L.st_cp_dst.upload(std::vector<int32_t>(dst.begin(), dst.begin() + std::ptrdiff_t(cut)));
+    }
+    if (cut < dst.size()) {
+        L.lat_cp_off.upload(lat_off);
+        L.lat_cp_dst.upload(std::vector<int32_t>(dst.begin() + std::ptrdiff_t(cut), dst.end()));
+    }
+}
 
 static Session* create_session(const egg_b200_session_desc& d)
 {
@@ -1281,6 +1316,7 @@ static Session* create_session(const egg_b200_session_desc& d)
     S->variant = 0;
     set_tiles(*S, *S, variant_shape(*S, 0));
     S->lat_node.upload(lat_node);
+    upload_copies(*S, sh_src, sh_dst, st_slot, lat_node);
     S->st_slot.upload(st_slot);
     S->st_off.upload(st_off);
     if (S->n_constrained) {
@@ -1519,6 +1555,7 @@ static StoredPatch2 stored_view(LevelData& S)
     sp.arena = (S.n_bspline || S.n_composite) ? S.arena.p : nullptr;
     sp.seeds = S.n_bspline ? S.seeds.p : nullptr;
     sp.soft = soft_view(S);
+    sp.copies = Copies {S.st_cp_off.p, S.st_cp_dst.p};
     return sp;
 }
 
@@ -1552,8 +1589,8 @@ static void launch_stored(Session& S, LevelData& L, const double* xin, double* x
                          L.st_wstride, L.st_wt.p, L.st_wtstride,
                          L.n_constrained ? L.st_etag.p : nullptr, L.n_constrained ? L.st_epar.p : nullptr,
                          cold ? 1 : 0, soft_view(L), L.n_bspline ? L.arena.p : nullptr,
-                         L.n_bspline ? L.seeds.p : nullptr};
-        const Lattice3 lat {L.n_lat, L.lat_node.p};
+                         L.n_bspline ? L.seeds.p : nullptr, Copies {L.st_cp_off.p, L.st_cp_dst.p}};
+        const Lattice3 lat {L.n_lat, L.lat_node.p, Copies {L.lat_cp_off.p, L.lat_cp_dst.p}};
         const int nb = L.n_stored ? int(grid) : 0;
         const unsigned all = unsigned(nb + (L.n_lat + kLatDofs - 1) / kLatDofs);
         const size_t sm = L.n_lat ? size_t(3 * WinLat3::N) * sizeof(double) : 0;
@@ -1759,8 +1796,6 @@ template <int KIND> static void launch_report(Session& S, const double* x, doubl
     }
 }
 
-// One block-Jacobi sweep xin -> xout (broadcast of the read buffer, then the
-// interior tiles and the stored-patch DOFs).
 // One relaxation of level L (or its gradient, gout): the interior tiles and
 // the stored-patch DOFs read the same snapshot and write disjoint slots, so
 // the stored-patch kernel forks onto the side stream beside the tiles.
@@ -1781,10 +1816,12 @@ static void relax_level(Session& S, LevelData& L, const double* xin, double* xou
     }
 }
 
+// One block-Jacobi sweep xin -> xout.  The copies of shared nodes agree with
+// their owners in xin, and (relaxed DOFs write theirs, the others' were equal
+// in both buffers) in xout.
 template <int KIND>
 static void sweep_once(Session& S, double* xin, double* xout, double delta, double omega, bool cold = false)
 {
-    launch_broadcast(S, S, xin);
     relax_level<KIND>(S, S, xin, xout, nullptr, delta, omega, nullptr, cold);
     S.updates += S.n_interior + S.n_stored + S.n_lat;
 }
@@ -1821,7 +1858,6 @@ static Session::ChunkGraph& chunk_graph(Session& S, int k, bool per_mesh, double
             sweep_once<KIND>(S, a, b, delta, omega);
             std::swap(a, b);
         }
-        launch_broadcast(S, S, a);
         launch_report<KIND>(S, a, delta, per_mesh, S.red_tmp.p);
     } catch (...) {
         cudaStreamEndCapture(S.stream, &graph);
@@ -1858,6 +1894,7 @@ template <int KIND> static void run_impl(Session& S, int n_sweeps, double delta,
     const size_t bytes = size_t(S.nstore) * S.dim * sizeof(double);
     double* xin = S.X(S.cur);
     double* xout = S.X(1 - S.cur);
+    launch_broadcast(S, S, xin);
     S.timed(kKCopy, [&] { EGG_CK(cudaMemcpyAsync(xout, xin, bytes, cudaMemcpyDeviceToDevice, S.stream)); });
     // Whole report chunks replay a captured graph (not while profiling, which
     // times every kernel with its own events).
@@ -1885,7 +1922,6 @@ template <int KIND> static void run_impl(Session& S, int n_sweeps, double delta,
         }
         sweep_once<KIND>(S, xin, xout, delta, omega, s == 0);
         if ((s + 1) % k == 0 || s == n_sweeps - 1) {
-            launch_broadcast(S, S, xout);
             launch_report<KIND>(S, xout, delta, per_mesh, slot);
             ++ridx;
         }
