@@ -53,44 +53,50 @@ struct Transfer {
     int64_t n_parent, n_coarse;
 };
 
+// Restriction in one launch: the injected positions into xc, rx (R x) and xs
+// (the level's other sweep buffer), and the full weighting of the parent
+// gradient gp onto free coarse nodes into tc (zero elsewhere).  The parent's
+// copies of shared nodes agree with their owners, so the coarse ones do too.
+// Interior coarse nodes read only their own block; interface coarse nodes
+// (listed in `iface`, with `iface_src[node * 3^D + e]` giving the parent slot of
+// stencil entry e, or -1 for an unused entry) read across the face.
+//
+// A coarse level is a few thousand nodes and its kernels take 3 to 6 us, most
+// of it launch and drain: what used to be two kernels, a broadcast and two
+// copies here, a clear and a difference around the coarse gradient, and a
+// difference, a prolongation and an update on the way up is now one launch
+// each way (513^2, 4 V(2,2) cycles on 9 levels: 140
+// of these launches, now 72; the whole pass 3.39 -> 2.49 ms).
 template <int D>
-__global__ void inject_kernel(Transfer t, const double* __restrict__ xp, double* __restrict__ xc)
+__global__ void restrict_kernel(Transfer t, const double* __restrict__ xp, double* __restrict__ xc,
+                                double* __restrict__ rx, double* __restrict__ xs, const double* __restrict__ gp,
+                                double* __restrict__ tc, const uint8_t* __restrict__ cfree,
+                                const int32_t* __restrict__ iface_slot, const int32_t* __restrict__ iface_src,
+                                int64_t n_iface)
 {
+    constexpr int NO = D == 2 ? 9 : 27;
     for (int64_t c = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; c < t.n_coarse;
          c += int64_t(gridDim.x) * blockDim.x) {
         const int b = find_block(t.coarse, t.nb, c);
         const BlockInfo cb = t.coarse[b], pb = t.parent[b];
         int I[3];
         unravel3(c - cb.off, cb.n, I);
-        const int64_t p = pb.off + ravel3(pb.n, I[0] * t.factor[3 * b], I[1] * t.factor[3 * b + 1],
-                                          I[2] * t.factor[3 * b + 2]);
+        const int f[3] = {t.factor[3 * b], t.factor[3 * b + 1], t.factor[3 * b + 2]};
+        {
+            const int64_t p = pb.off + ravel3(pb.n, I[0] * f[0], I[1] * f[1], I[2] * f[2]);
 #pragma unroll
-        for (int k = 0; k < D; ++k) { xc[D * c + k] = xp[D * p + k]; }
-    }
-}
-
-// Full weighting of the parent gradient onto free coarse nodes.  Interior
-// coarse nodes read only their own block; interface coarse nodes (listed in
-// `iface`, with `iface_src[node * 3^D + e]` giving the parent slot of
-// stencil entry e, or -1 for an unused entry) read across the face.
-template <int D>
-__global__ void full_weight_kernel(Transfer t, const double* __restrict__ gp, double* __restrict__ tc,
-                                   const uint8_t* __restrict__ cfree, const int32_t* __restrict__ iface_slot,
-                                   const int32_t* __restrict__ iface_src, int64_t n_iface)
-{
-    constexpr int NO = D == 2 ? 9 : 27;
-    for (int64_t c = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; c < t.n_coarse;
-         c += int64_t(gridDim.x) * blockDim.x) {
+            for (int k = 0; k < D; ++k) {
+                const double v = xp[D * p + k];
+                xc[D * c + k] = v;
+                rx[D * c + k] = v;
+                xs[D * c + k] = v;
+            }
+        }
         if (cfree[c] == 2) { continue; }  // free interface node: table path below
         double acc[D];
 #pragma unroll
         for (int k = 0; k < D; ++k) { acc[k] = 0.0; }
         if (cfree[c] == 1) {  // free interior node
-            const int b = find_block(t.coarse, t.nb, c);
-            const BlockInfo cb = t.coarse[b], pb = t.parent[b];
-            int I[3];
-            unravel3(c - cb.off, cb.n, I);
-            const int f[3] = {t.factor[3 * b], t.factor[3 * b + 1], t.factor[3 * b + 2]};
             for (int e = 0; e < NO; ++e) {
                 int rem = e;
                 int F[3] = {I[0] * f[0], I[1] * f[1], I[2] * f[2]};
@@ -142,12 +148,21 @@ __global__ void full_weight_kernel(Transfer t, const double* __restrict__ gp, do
     }
 }
 
-// Multilinear prolongation of a coarse correction onto every parent node.
-template <int D>
-__global__ void prolong_kernel(Transfer t, const double* __restrict__ cc, double* __restrict__ cp)
+// Multilinear prolongation of the coarse correction xc - rx onto the masked
+// parent nodes: x += it (ADD), or out = it, zero off the mask.
+template <int D, bool ADD>
+__global__ void prolong_kernel(Transfer t, const double* __restrict__ xc, const double* __restrict__ rx,
+                               const uint8_t* __restrict__ mask, double* __restrict__ out)
 {
     for (int64_t p = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; p < t.n_parent;
          p += int64_t(gridDim.x) * blockDim.x) {
+        if (!mask[p]) {
+            if constexpr (!ADD) {
+#pragma unroll
+                for (int k = 0; k < D; ++k) { out[D * p + k] = 0.0; }
+            }
+            continue;
+        }
         const int b = find_block(t.parent, t.nb, p);
         const BlockInfo cb = t.coarse[b], pb = t.parent[b];
         int J[3];
@@ -178,10 +193,10 @@ __global__ void prolong_kernel(Transfer t, const double* __restrict__ cc, double
             if (!valid) { continue; }
             const int64_t q = cb.off + ravel3(cb.n, C[0], C[1], C[2]);
 #pragma unroll
-            for (int k = 0; k < D; ++k) { acc[k] += w0 * cc[D * q + k]; }
+            for (int k = 0; k < D; ++k) { acc[k] += w0 * (xc[D * q + k] - rx[D * q + k]); }
         }
 #pragma unroll
-        for (int k = 0; k < D; ++k) { cp[D * p + k] = acc[k]; }
+        for (int k = 0; k < D; ++k) { out[D * p + k] = ADD ? out[D * p + k] + acc[k] : acc[k]; }
     }
 }
 
@@ -195,22 +210,6 @@ __global__ void masked_axpy_kernel(double* out, const double* x, const double* c
         const double ai = (mask == nullptr || mask[i]) ? a : 0.0;
 #pragma unroll
         for (int k = 0; k < D; ++k) { out[D * i + k] = x[D * i + k] + ai * c[D * i + k]; }
-    }
-}
-
-template <int D> __global__ void zero_unmasked_kernel(double* buf, const uint8_t* mask, int64_t n)
-{
-    for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
-        if (mask[i]) { continue; }
-#pragma unroll
-        for (int k = 0; k < D; ++k) { buf[D * i + k] = 0.0; }
-    }
-}
-
-__global__ void vec_sub_kernel(double* out, const double* a, const double* b, int64_t n)
-{
-    for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
-        out[i] = a[i] - b[i];
     }
 }
 
