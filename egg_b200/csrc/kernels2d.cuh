@@ -6,10 +6,12 @@
 // or to the block's own refreshed copies of shared interface nodes.
 //
 // One block-Jacobi sweep (src/sweep.hpp:1938 jacobi_sweep_once) is
-//   broadcast_kernel     owner -> non-owner copies on the read buffer
-//   interior_tile_kernel structured-interior DOFs (patch synthesized, W_inv = I)
-//   stored_patch_kernel  every other moving DOF (ragged stored patch)
-// Both sweep kernels read X_in (frozen snapshot) and write X_out.
+//   interior_fp64_kernel structured-interior DOFs (patch synthesized, W_inv = I;
+//                        mixed precision: interior_x2_kernel)
+//   stored_patch_kernel  every other moving DOF (ragged stored patch); it also
+//                        writes the DOF's copies in other blocks
+// Both read X_in (frozen snapshot) and write X_out.  Nodes that no DOF moves
+// keep the copies that both buffers start with (broadcast2_kernel).
 #pragma once
 
 #include "entity2.cuh"
@@ -686,7 +688,15 @@ constexpr int64_t kStoredFillThreads3 = 148 * 16384;
 // (gradient, contracted Hessian, energy; then each line-search trial) and
 // reduce across the group, so a ragged patch of 16-64 gathered samples can be
 // a few rounds of parallel work instead of one thread's serial loop.
-template <int KIND, int G, bool CON>
+//
+// A sweep of a small mesh is one such chain (gathers, metric, reductions,
+// projections, trials) in a few warps per SM, so its latency is what counts.
+// CON says which entity code is compiled in: 0 none (no DOF is constrained),
+// 1 all but B-splines and composites, 2 all of it.  The B-spline Newton solves
+// alone take the kernel from 304 to 1408 bytes of stack and from 122 to 164
+// registers, which every DOF on an arc paid for (5 x 129^2 disk sliding on
+// arcs, 40 sweeps: 1097 us with one class for all entities, now 918).
+template <int KIND, int G, int CON>
 __global__ void stored_patch_kernel(StoredPatch2 sp, const double2* __restrict__ Xin,
                                     double2* __restrict__ Xout, const double2* __restrict__ tau,
                                     double delta, double omega, double2* __restrict__ grad_out)
@@ -764,14 +774,13 @@ __global__ void stored_patch_kernel(StoredPatch2 sp, const double2* __restrict__
         // A trimmed curve after the first sweep of a run call searches in its
         // parameter instead (src/sweep.hpp:1718-1876): trials q* + alpha dq,
         // clamped onto the trim and evaluated on the curve.
-        // CON = false (a level without constrained DOFs) compiles none of it.
         const double* er = sp.epar + (etag != 0 ? d * EGG_B200_ENTITY_FIELDS : 0);
         const bool warm_arc = is_tcurve(etag) && !sp.cold;
         // B-spline DOFs carry a seed (their last foot parameter): every seeded
         // projection starts its Newton solve there and stores its result
         // (src/sweep.hpp:1219-1265).
-        const bool bsp = etag == EGG_B200_TAG_BSPLINE;
-        const bool comp = etag == EGG_B200_TAG_COMPOSITE;
+        const bool bsp = CON == 2 && etag == EGG_B200_TAG_BSPLINE;
+        const bool comp = CON == 2 && etag == EGG_B200_TAG_COMPOSITE;
         const double* cslice = comp ? sp.arena + int64_t(er[6]) : nullptr;  // the path's arena slice
         const double* crec = comp ? cslice + int64_t(er[1]) : nullptr;
         const int cseg = comp ? int(er[0]) : 0;

@@ -4,13 +4,13 @@
 // per node, packed back to back (same conventions as the 2D store).
 //
 // interior3_kernel: one CTA = a TI x TJ x TK tile of structured-interior DOFs;
-// the (TI+2)(TJ+2)(TK+2) node window is staged in shared memory and each thread
-// relaxes one DOF over its 64-occurrence patch (8 cells x 8 corner samples,
-// src/structured_patch.hpp:89-258): for each of its four roles the 8 samples
-// that move it contribute gradient and contracted Hessian (metric3.cuh), the
-// 32 samples that do not move it contribute a constant energy and min det;
-// then the 3x3 Newton step, <= 10 halvings on the 32 moving samples, omega
-// blend (src/sweep.hpp:1534-1650).
+// the (TI+2)(TJ+2)(TK+2) node window is staged in shared memory (with its fp32
+// forward edges in the mixed path) and each thread relaxes one DOF over its
+// 64-occurrence patch (8 cells x 8 corner samples,
+// src/structured_patch.hpp:89-258): dof3.cuh evaluates the 32 samples that
+// move it, grouped by the edge that moves; the 32 that do not move it only
+// rule a step out, from per-cell bits; then the 3x3 Newton step, <= 10 halvings
+// on the moving samples, omega blend (src/sweep.hpp:1534-1650).
 #pragma once
 
 #include "dof3.cuh"

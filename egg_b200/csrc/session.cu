@@ -1620,7 +1620,7 @@ static void launch_stored(Session& S, LevelData& L, const double* xin, double* x
     const auto* t2 = reinterpret_cast<const double2*>(tau);
     auto* g2 = reinterpret_cast<double2*>(gout);
     auto go2 = [&](auto con) {
-        constexpr bool C = decltype(con)::value;
+        constexpr int C = decltype(con)::value;
         switch (G) {
         case 32: stored_patch_kernel<KIND, 32, C><<<grid, 128, 0, st>>>(sp, x2, o2, t2, delta, omega, g2); break;
         case 8: stored_patch_kernel<KIND, 8, C><<<grid, 128, 0, st>>>(sp, x2, o2, t2, delta, omega, g2); break;
@@ -1629,12 +1629,16 @@ static void launch_stored(Session& S, LevelData& L, const double* xin, double* x
         }
     };
     // Levels without constrained DOFs (every coarse FAS level, most meshes)
-    // launch the instantiation that carries no entity code.
+    // launch the instantiation that carries no entity code, levels whose
+    // entities are all closed-form or trimmed curves the one without the
+    // B-spline and composite code.
     S.timed(kKStored, [&] {
-        if (L.n_constrained) {
-            go2(std::true_type {});
+        if (!L.n_constrained) {
+            go2(std::integral_constant<int, 0> {});
+        } else if (!L.n_bspline && !L.n_composite) {
+            go2(std::integral_constant<int, 1> {});
         } else {
-            go2(std::false_type {});
+            go2(std::integral_constant<int, 2> {});
         }
     });
 }
