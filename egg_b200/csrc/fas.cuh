@@ -32,12 +32,13 @@ __device__ __forceinline__ int find_block(const BlockInfo* blocks, int nb, int64
     return lo;
 }
 
+// f < 2^31 (the store's limit): 32-bit divisions, a third of the 64-bit ones.
 __device__ __forceinline__ void unravel3(int64_t f, const int32_t n[3], int I[3])
 {
-    I[2] = int(f % n[2]);
-    f /= n[2];
-    I[1] = int(f % n[1]);
-    I[0] = int(f / n[1]);
+    const uint32_t g = uint32_t(f), n2 = uint32_t(n[2]), n1 = uint32_t(n[1]), h = g / n2;
+    I[2] = int(g - h * n2);
+    I[0] = int(h / n1);
+    I[1] = int(h - uint32_t(I[0]) * n1);
 }
 
 __device__ __forceinline__ int64_t ravel3(const int32_t n[3], int i, int j, int k)

@@ -935,17 +935,56 @@ __device__ __forceinline__ bool block_reduce(Comp& acc, double& mn)
     return lane == 0;
 }
 
-// Block reduction into partial slot blockIdx.y * gridDim.x + blockIdx.x
-// (blockIdx.y = segment of a segmented reduction, 0 otherwise).
-__device__ __forceinline__ void block_reduce_store(Comp acc, double mn, double* part_s,
-                                                   double* part_c, double* part_m)
+// Where a whole-store reduction leaves its result; ticket counts the CTAs that
+// have stored their partials (zero between launches; NULL: a segmented
+// reduction, or one that reduce_finalize_kernel ends).
+struct ReduceOut {
+    double* e = nullptr;
+    double* m = nullptr;
+    unsigned* ticket = nullptr;
+};
+
+// The partials summed in a fixed order by one CTA: out_e = energy, out_m = min det.
+__device__ __forceinline__ void reduce_partials(const double* part_s, const double* part_c, const double* part_m,
+                                                int n, double* out_e, double* out_m)
 {
+    Comp acc {0.0, 0.0};
+    double mn = INFINITY;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        acc = comp_merge(acc, Comp {__ldcg(part_s + i), __ldcg(part_c + i)});
+        mn = fmin(mn, __ldcg(part_m + i));
+    }
+    if (block_reduce(acc, mn)) {
+        *out_e = acc.s + acc.c;
+        *out_m = mn;
+    }
+}
+
+// Block reduction into partial slot blockIdx.y * gridDim.x + blockIdx.x
+// (blockIdx.y = segment of a segmented reduction, 0 otherwise).  The last CTA to
+// store sums the partials, which was a launch of its own (513^2, 4 FAS cycles
+// with 12 reductions: 2507 -> 2458 us).  Which CTA is last does not change the
+// order of the sum.
+__device__ __forceinline__ void block_reduce_store(Comp acc, double mn, double* part_s, double* part_c,
+                                                   double* part_m, ReduceOut out)
+{
+    __shared__ bool last;
     if (block_reduce(acc, mn)) {
         const int64_t slot = int64_t(blockIdx.y) * gridDim.x + blockIdx.x;
         part_s[slot] = acc.s;
         part_c[slot] = acc.c;
         part_m[slot] = mn;
+        if (out.ticket != nullptr) {
+            __threadfence();
+            last = atomicAdd(out.ticket, 1u) == gridDim.x - 1;
+        }
     }
+    if (out.ticket == nullptr) { return; }
+    __syncthreads();
+    if (!last) { return; }
+    __threadfence();
+    reduce_partials(part_s, part_c, part_m, int(gridDim.x), out.e, out.m);
+    if (threadIdx.x == 0) { *out.ticket = 0u; }
 }
 
 // Item range of this CTA row: segment blockIdx.y of `seg` (prefix offsets),
@@ -971,7 +1010,7 @@ struct EnergyStructured2 {
 template <int KIND>
 __global__ void energy_structured2_kernel(EnergyStructured2 es, const double2* __restrict__ X,
                                           double delta, double* part_s, double* part_c,
-                                          double* part_m)
+                                          double* part_m, ReduceOut out = {})
 {
     Comp acc {0.0, 0.0};
     double mn = INFINITY;
@@ -989,8 +1028,8 @@ __global__ void energy_structured2_kernel(EnergyStructured2 es, const double2* _
             }
         }
         const BlockInfo bi = es.blocks[lo];
-        const int64_t lc = c - es.cell_off[lo];
-        const int cw = bi.n[1] - 1;
+        const uint32_t lc = uint32_t(c - es.cell_off[lo]);  // a store holds < 2^31 nodes
+        const uint32_t cw = uint32_t(bi.n[1] - 1);
         const int i = int(lc / cw), j = int(lc % cw);
         const int64_t base = bi.off + int64_t(i) * bi.n[1] + j;
         const double2 p[4] = {X[base], X[base + 1], X[base + bi.n[1]], X[base + bi.n[1] + 1]};
@@ -1005,7 +1044,7 @@ __global__ void energy_structured2_kernel(EnergyStructured2 es, const double2* _
             mn = fmin(mn, detA);
         }
     }
-    block_reduce_store(acc, mn, part_s, part_c, part_m);
+    block_reduce_store(acc, mn, part_s, part_c, part_m, out);
 }
 
 struct EnergyStored2 {
@@ -1024,7 +1063,7 @@ struct EnergyStored2 {
 
 template <int KIND>
 __global__ void energy_stored2_kernel(EnergyStored2 es, const double2* __restrict__ X, double delta,
-                                      double* part_s, double* part_c, double* part_m)
+                                      double* part_s, double* part_c, double* part_m, ReduceOut out = {})
 {
     Comp acc {0.0, 0.0};
     double mn = INFINITY;
@@ -1038,23 +1077,15 @@ __global__ void energy_stored2_kernel(EnergyStored2 es, const double2* __restric
         comp_add(acc, es.wt[i * es.wt_stride] * mu_value<double>(KIND, t, delta));
         mn = fmin(mn, detA);
     }
-    block_reduce_store(acc, mn, part_s, part_c, part_m);
+    block_reduce_store(acc, mn, part_s, part_c, part_m, out);
 }
 
-// Single-CTA final pass over the partials, fixed order: out[0] = energy, out[1] = min det.
-__global__ void reduce_finalize_kernel(const double* part_s, const double* part_c,
-                                       const double* part_m, int n, double* out_e, double* out_m)
+// Single-CTA final pass over the partials, in the order of the sum that
+// block_reduce_store ends with (256 threads).
+__global__ void reduce_finalize_kernel(const double* part_s, const double* part_c, const double* part_m, int n,
+                                       double* out_e, double* out_m)
 {
-    Comp acc {0.0, 0.0};
-    double mn = INFINITY;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        acc = comp_merge(acc, Comp {part_s[i], part_c[i]});
-        mn = fmin(mn, part_m[i]);
-    }
-    if (block_reduce(acc, mn)) {
-        *out_e = acc.s + acc.c;
-        *out_m = mn;
-    }
+    reduce_partials(part_s, part_c, part_m, n, out_e, out_m);
 }
 
 // Adds the whole-sample directional total to a finished energy report

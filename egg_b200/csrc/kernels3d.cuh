@@ -705,7 +705,7 @@ __global__ void broadcast3_kernel(double* __restrict__ X, const int32_t* __restr
 // Energy / min det over the canonical cell stencil of the blocks (3D).
 template <int KIND>
 __global__ void energy_structured3_kernel(EnergyStructured2 es, const double* __restrict__ X, double delta,
-                                          double* part_s, double* part_c, double* part_m)
+                                          double* part_s, double* part_c, double* part_m, ReduceOut out = {})
 {
     Comp acc {0.0, 0.0};
     double mn = INFINITY;
@@ -723,9 +723,9 @@ __global__ void energy_structured3_kernel(EnergyStructured2 es, const double* __
             }
         }
         const BlockInfo bi = es.blocks[lo];
-        const int64_t lc = c - es.cell_off[lo];
-        const int c1 = bi.n[1] - 1, c2 = bi.n[2] - 1;
-        const int i = int(lc / (int64_t(c1) * c2)), j = int((lc / c2) % c1), k = int(lc % c2);
+        const uint32_t lc = uint32_t(c - es.cell_off[lo]);  // a store holds < 2^31 nodes
+        const uint32_t c1 = uint32_t(bi.n[1] - 1), c2 = uint32_t(bi.n[2] - 1), ij = lc / c2;
+        const int i = int(ij / c1), j = int(ij % c1), k = int(lc % c2);
         const int32_t base = int32_t(bi.off + (int64_t(i) * bi.n[1] + j) * bi.n[2] + k);
         int32_t nd[8];
 #pragma unroll
@@ -743,7 +743,7 @@ __global__ void energy_structured3_kernel(EnergyStructured2 es, const double* __
             mn = fmin(mn, detA);
         }
     }
-    block_reduce_store(acc, mn, part_s, part_c, part_m);
+    block_reduce_store(acc, mn, part_s, part_c, part_m, out);
 }
 
 struct EnergyStored3 {
@@ -764,7 +764,7 @@ struct EnergyStored3 {
 
 template <int KIND>
 __global__ void energy_stored3_kernel(EnergyStored3 es, const double* __restrict__ X, double delta, double* part_s,
-                                      double* part_c, double* part_m)
+                                      double* part_c, double* part_m, ReduceOut out = {})
 {
     Comp acc {0.0, 0.0};
     double mn = INFINITY;
@@ -781,7 +781,7 @@ __global__ void energy_stored3_kernel(EnergyStored3 es, const double* __restrict
         comp_add(acc, es.wt[i * es.wt_stride] * mu3_value<double>(KIND, t, delta, dd));
         mn = fmin(mn, detA);
     }
-    block_reduce_store(acc, mn, part_s, part_c, part_m);
+    block_reduce_store(acc, mn, part_s, part_c, part_m, out);
 }
 
 // Device metric probe (tests): mu, gradient over vec(T) (9) and the contracted

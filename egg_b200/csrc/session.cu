@@ -246,6 +246,7 @@ struct Session : LevelData {
     // reductions
     int red_grid = 0;
     DevBuf<double> part;      // [3 * red_grid]
+    DevBuf<unsigned> red_ticket;  // CTAs of a running reduction that are done (0 between launches)
     DevBuf<double> red_out;   // [2 * capacity]
     DevBuf<double> red_tmp;   // [2 * n_seg or 2]: report slot written inside a captured chunk
     // batch: several independent meshes packed into one store
@@ -1382,6 +1383,7 @@ static Session* create_session(const egg_b200_session_desc& d)
     S->cur = 0;
     S->red_grid = 148 * 4;
     S->part.alloc(3 * size_t(S->red_grid));
+    S->red_ticket.upload(std::vector<unsigned> {0u});
     S->red_out.alloc(2);
     EGG_CK(cudaDeviceSynchronize());
     return S.release();
@@ -1674,6 +1676,7 @@ template <int KIND> static void launch_reduce(Session& S, const double* x, doubl
     double* ps = S.part.p;
     double* pc = ps + S.red_grid;
     double* pm = pc + S.red_grid;
+    const ReduceOut out {out_e, out_m, S.red_ticket.p};
     const auto* X2 = reinterpret_cast<const double2*>(x);
     if (S.es_struct) {
         EnergyStructured2 es;
@@ -1687,18 +1690,18 @@ template <int KIND> static void launch_reduce(Session& S, const double* x, doubl
         es.wt_stride = S.es_wtstride;
         if (S.dim == 3) {
             S.timed(kKReduce, [&] {
-                energy_structured3_kernel<KIND><<<S.red_grid, 256, 0, S.stream>>>(es, x, delta, ps, pc, pm);
+                energy_structured3_kernel<KIND><<<S.red_grid, 256, 0, S.stream>>>(es, x, delta, ps, pc, pm, out);
             });
         } else {
             S.timed(kKReduce, [&] {
-                energy_structured2_kernel<KIND><<<S.red_grid, 256, 0, S.stream>>>(es, X2, delta, ps, pc, pm);
+                energy_structured2_kernel<KIND><<<S.red_grid, 256, 0, S.stream>>>(es, X2, delta, ps, pc, pm, out);
             });
         }
     } else if (S.dim == 3) {
         EnergyStored3 es {S.es_ns,  S.es_gc.p, S.es_gn0.p,    S.es_gn1.p, S.es_gn2.p,     S.es_s0.p,
                           S.es_s1.p, S.es_s2.p, S.es_W.p, S.es_wstride, S.es_wt.p, S.es_wtstride};
         S.timed(kKReduce, [&] {
-            energy_stored3_kernel<KIND><<<S.red_grid, 256, 0, S.stream>>>(es, x, delta, ps, pc, pm);
+            energy_stored3_kernel<KIND><<<S.red_grid, 256, 0, S.stream>>>(es, x, delta, ps, pc, pm, out);
         });
     } else {
         EnergyStored2 es;
@@ -1713,10 +1716,9 @@ template <int KIND> static void launch_reduce(Session& S, const double* x, doubl
         es.wt = S.es_wt.p;
         es.wt_stride = S.es_wtstride;
         S.timed(kKReduce, [&] {
-            energy_stored2_kernel<KIND><<<S.red_grid, 256, 0, S.stream>>>(es, X2, delta, ps, pc, pm);
+            energy_stored2_kernel<KIND><<<S.red_grid, 256, 0, S.stream>>>(es, X2, delta, ps, pc, pm, out);
         });
     }
-    S.timed(kKFinal, [&] { reduce_finalize_kernel<<<1, 1024, 0, S.stream>>>(ps, pc, pm, S.red_grid, out_e, out_m); });
     launch_soft_energy(S, x, out_e);
 }
 
@@ -2041,7 +2043,7 @@ static void energy_noalloc_impl(Session& S, double delta, int grid, double* scra
         energy_stored2_kernel<KIND><<<grid, 256, 0, S.stream>>>(es, X2, delta, ps, pc, pm);
     }
     EGG_CK(cudaGetLastError());
-    reduce_finalize_kernel<<<1, 1024, 0, S.stream>>>(ps, pc, pm, grid, out, out + 1);
+    reduce_finalize_kernel<<<1, 256, 0, S.stream>>>(ps, pc, pm, grid, out, out + 1);
     EGG_CK(cudaGetLastError());
     S.launches += 2;
     if (S.es_dir_n) {
