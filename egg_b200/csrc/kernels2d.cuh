@@ -41,11 +41,6 @@ struct __align__(16) Tile2 {
     int32_t pad[2];
 };
 
-// Relative threshold of the fp64 guard in mixed precision: a sample whose
-// |det A| < kGuard * |a0| |a1| (sine of the corner angle below 1e-3) is
-// re-evaluated in fp64.
-constexpr double kGuard = 1e-3;
-
 __device__ __forceinline__ double2 ld2(const double2* p) { return *p; }
 
 // ---------------------------------------------------------------------------

@@ -50,6 +50,11 @@ template <> struct Tol<float> {
     static constexpr float znorm = 1e-7f;
 };
 
+// Relative threshold of the fp64 guard in mixed precision: a sample whose
+// |det A| < kGuard * |a0| |a1| (sine of the corner angle below 1e-3) is
+// re-evaluated in fp64.
+constexpr double kGuard = 1e-3;
+
 template <class R> EGG_HD R det2(const R t[4]) { return t[0] * t[3] - t[1] * t[2]; }
 
 // f(D) and its first two derivatives for the shape-type objectives.

@@ -64,6 +64,16 @@ X2_HD float2 fma2(float2 a, float2 b, float2 c)
 #endif
 }
 
+// a * b rounded by itself: never contracted into a sum
+X2_HD float fmul_rn(float a, float b)
+{
+#if defined(__CUDA_ARCH__)
+    return __fmul_rn(a, b);
+#else
+    return a * b;
+#endif
+}
+
 // a - b: b * (-1) + a is exact before its one rounding, so this equals the
 // correctly rounded difference.
 X2_HD float2 sub2(float2 a, float2 b) { return fma2(b, p2(-1.0f), a); }
