@@ -163,6 +163,10 @@ struct LevelData {
     DevBuf<int32_t> lat_node;
     // the copies of the stored and the lattice DOFs (empty without shared nodes)
     DevBuf<int32_t> st_cp_off, st_cp_dst, lat_cp_off, lat_cp_dst;
+    // owner -> copy entries that a tile's DOF takes part in (none on a grid
+    // whose blocks meet in faces only)
+    int64_t n_tile_cp = 0;
+    DevBuf<int32_t> tile_cp_src, tile_cp_dst;
     int64_t n_stored = 0;
     DevBuf<int32_t> st_slot, st_gc, st_gn0, st_gn1, st_gn2, st_role;
     DevBuf<int64_t> st_off;
@@ -570,7 +574,9 @@ static void set_tiles(Session& S, LevelData& L, Variant v)
 #include "lattice_host.inc"
 
 // Copies tables of a level's stored and lattice DOFs from its owner -> copy
-// pairs.
+// pairs, and the pairs with a slot that a tile relaxes: blocks that overlap
+// share nodes that lie strictly inside one of them.  A tile writes its own slot
+// alone, so relax_level refreshes those copies behind it.
 static void upload_copies(LevelData& L, const std::vector<int32_t>& sh_src, const std::vector<int32_t>& sh_dst,
                           const std::vector<int32_t>& st_slot, const std::vector<int32_t>& lat_node)
 {
@@ -585,10 +591,18 @@ static void upload_copies(LevelData& L, const std::vector<int32_t>& sh_src, cons
     }
     for (size_t d = 0; d < ns + nl; ++d) { off[d + 1] += off[d]; }
     std::vector<int32_t> at(off.begin(), off.end() - 1), dst(size_t(off.back()));
+    std::vector<int32_t> tile_src, tile_dst;
     for (size_t e = 0; e < sh_src.size(); ++e) {
         const int32_t d = of[size_t(sh_src[e])];
         if (d >= 0) { dst[size_t(at[size_t(d)]++)] = sh_dst[e]; }
+        if (L.active_h[size_t(sh_src[e])] || L.active_h[size_t(sh_dst[e])]) {
+            tile_src.push_back(sh_src[e]);
+            tile_dst.push_back(sh_dst[e]);
+        }
     }
+    L.n_tile_cp = int64_t(tile_src.size());
+    L.tile_cp_src.upload(tile_src);
+    L.tile_cp_dst.upload(tile_dst);
     const size_t cut = size_t(off[ns]);
     std::vector<int32_t> lat_off(off.begin() + std::ptrdiff_t(ns), off.end());
     for (int32_t& v : lat_off) { v -= int32_t(cut); }
@@ -1645,17 +1659,22 @@ static void launch_stored(Session& S, LevelData& L, const double* xin, double* x
     });
 }
 
+static void launch_copies(Session& S, const int32_t* src, const int32_t* dst, int64_t n, double* x)
+{
+    if (n == 0) { return; }
+    const unsigned grid = unsigned(std::min<int64_t>((n + 255) / 256, 148 * 8));
+    S.timed(kKBroadcast, [&] {
+        if (S.dim == 3) {
+            broadcast3_kernel<<<grid, 256, 0, S.stream>>>(x, src, dst, n);
+        } else {
+            broadcast2_kernel<<<grid, 256, 0, S.stream>>>(reinterpret_cast<double2*>(x), src, dst, n);
+        }
+    });
+}
+
 static void launch_broadcast(Session& S, LevelData& L, double* x)
 {
-    if (L.nshare == 0) { return; }
-    const unsigned grid = unsigned(std::min<int64_t>((L.nshare + 255) / 256, 148 * 8));
-    if (S.dim == 3) {
-        S.timed(kKBroadcast, [&] { broadcast3_kernel<<<grid, 256, 0, S.stream>>>(x, L.sh_src.p, L.sh_dst.p, L.nshare); });
-        return;
-    }
-    S.timed(kKBroadcast, [&] {
-        broadcast2_kernel<<<grid, 256, 0, S.stream>>>(reinterpret_cast<double2*>(x), L.sh_src.p, L.sh_dst.p, L.nshare);
-    });
+    launch_copies(S, L.sh_src.p, L.sh_dst.p, L.nshare, x);
 }
 
 // The whole-sample directional total, added onto *out_e (no-op without one).
@@ -1820,11 +1839,12 @@ static void relax_level(Session& S, LevelData& L, const double* xin, double* xou
         launch_interior<KIND>(S, L, xin, xout, tau, delta, omega, gout);
         launch_stored<KIND>(S, L, xin, xout, tau, delta, omega, gout, nullptr, cold);
     }
+    if (gout == nullptr) { launch_copies(S, L.tile_cp_src.p, L.tile_cp_dst.p, L.n_tile_cp, xout); }
 }
 
 // One block-Jacobi sweep xin -> xout.  The copies of shared nodes agree with
-// their owners in xin, and (relaxed DOFs write theirs, the others' were equal
-// in both buffers) in xout.
+// their owners in xin, and in xout: stored DOFs write theirs, relax_level
+// refreshes those of a tile's DOF, and the others' were equal in both buffers.
 template <int KIND>
 static void sweep_once(Session& S, double* xin, double* xout, double delta, double omega, bool cold = false)
 {
