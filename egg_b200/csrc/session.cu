@@ -301,6 +301,7 @@ struct Session : LevelData {
         }
         for (cudaEvent_t e : event_pool) { cudaEventDestroy(e); }
         if (side) { cudaStreamSynchronize(side); }
+        if (stream) { cudaStreamSynchronize(stream); }  // a failed transfer may still use pin
         if (fork_ev) { cudaEventDestroy(fork_ev); }
         if (join_ev) { cudaEventDestroy(join_ev); }
         if (side) { cudaStreamDestroy(side); }
@@ -308,7 +309,7 @@ struct Session : LevelData {
         for (cudaEvent_t e : xfer_ev) {
             if (e) { cudaEventDestroy(e); }
         }
-        if (pin) { cudaFreeHost(pin); }
+        if (pin) { egg_b200_pinned_release(pin); }
     }
 
     cudaEvent_t take_event()
@@ -2262,13 +2263,16 @@ struct egg_b200_session {
 };
 
 
-// Pinned staging for transfers from and to pageable memory.
+// Pinned staging for transfers from and to pageable memory, from the pool: a
+// page-locked allocation takes as long as several passes (37 MB: 15 ms).
 static void ensure_pin(Session& S)
 {
-    const size_t n = size_t(S.M) * S.dim;
-    if (!S.pin && n) {
-        EGG_CK(cudaHostAlloc(reinterpret_cast<void**>(&S.pin), n * sizeof(double), cudaHostAllocDefault));
-    }
+    const int64_t bytes = S.M * S.dim * int64_t(sizeof(double));
+    if (S.pin || bytes == 0) { return; }
+    void* p = nullptr;
+    const int rc = egg_b200_pinned_acquire(bytes, &p);
+    if (rc != EGG_B200_OK) { throw Error(rc, egg_b200_last_error()); }
+    S.pin = static_cast<double*>(p);
 }
 
 static void ensure_xfer(Session& S)
@@ -2284,26 +2288,49 @@ static void ensure_xfer(Session& S)
 
 static void reset_seeds(Session& S);
 
+// An array of a transfer that is worth a DMA of its own, straight from or to
+// the caller's memory: page-locked, and large.  A DMA costs some 2 us to queue
+// and finding out whether memory is page-locked another, what a host thread
+// copies 64 KB in; a batch of 1024 meshes of 9^2 spent 3.6 ms in them, 0.4 ms
+// through the staging.
+constexpr int64_t kDirectMin = 32768;  // reals
+static bool direct_copy(const double* p, int64_t len, int n_arrays)
+{
+    if (len == 0 || (len < kDirectMin && n_arrays > 1)) { return false; }
+    cudaPointerAttributes attr {};
+    const bool pinned = cudaPointerGetAttributes(&attr, p) == cudaSuccess && attr.type == cudaMemoryTypeHost;
+    cudaGetLastError();
+    return pinned;
+}
+
+// Calls f(m, lo, hi) for the parts of the concatenation [at[m], at[m + 1]) of
+// the arrays that lie in [a, b).
+template <class F> static void each_part(const std::vector<size_t>& at, size_t a, size_t b, F f)
+{
+    size_t m = size_t(std::upper_bound(at.begin(), at.end(), a) - at.begin()) - 1;
+    for (; m + 1 < at.size() && at[m] < b; ++m) {
+        const size_t lo = std::max(a, at[m]), hi = std::min(b, at[m + 1]);
+        if (lo < hi) { f(m, lo, hi); }
+    }
+}
+
 // Positions in global node order, given as n arrays one after another, into
-// every copy of the store.  Page-locked arrays: one DMA each straight from
-// them.  The others: host thread t stages its slice of the concatenation in
-// pinned memory and queues its H2D, so the DMA of early slices overlaps the
-// staging of later ones.
+// every copy of the store.  Large page-locked arrays: one DMA each straight
+// from them.  The others: host thread t stages its slice of the concatenation
+// in pinned memory and queues its H2D, one for what lies side by side, so the
+// DMA of early slices overlaps the staging of later ones.
 static void upload_X(Session& S, const double* const* X, const int64_t* len, int n)
 {
     const int D = S.dim;
     EGG_CK(cudaSetDevice(S.device));
     ensure_xfer(S);
     std::vector<size_t> at(size_t(n) + 1, 0);
-    std::vector<char> pinned(size_t(n), 0);
+    std::vector<char> direct(size_t(n), 0);
     size_t staged = 0;
     for (int m = 0; m < n; ++m) {
         at[size_t(m) + 1] = at[size_t(m)] + size_t(len[m]);
-        if (!len[m]) { continue; }
-        cudaPointerAttributes attr {};
-        pinned[size_t(m)] = cudaPointerGetAttributes(&attr, X[m]) == cudaSuccess && attr.type == cudaMemoryTypeHost;
-        cudaGetLastError();
-        if (pinned[size_t(m)]) {
+        direct[size_t(m)] = direct_copy(X[m], len[m], n);
+        if (direct[size_t(m)]) {
             EGG_CK(cudaMemcpyAsync(S.Xg.p + at[size_t(m)], X[m], size_t(len[m]) * sizeof(double),
                                    cudaMemcpyHostToDevice, S.stream));
         } else {
@@ -2316,16 +2343,24 @@ static void upload_X(Session& S, const double* const* X, const int64_t* len, int
         const int T = copy_threads(staged * sizeof(double));
         cudaError_t err[kMaxCopyThreads] = {};
         run_slices(T, [&](int t) {
-            const size_t a = slice_begin(total, t, T), b = slice_begin(total, t + 1, T);
             err[t] = cudaSetDevice(S.device);
-            size_t m = size_t(std::upper_bound(at.begin(), at.end(), a) - at.begin()) - 1;
-            for (; m < size_t(n) && at[m] < b; ++m) {
-                const size_t lo = std::max(a, at[m]), hi = std::min(b, at[m + 1]);
-                if (pinned[m] || hi <= lo || err[t] != cudaSuccess) { continue; }
+            size_t r0 = 0, r1 = 0;  // staged and not yet queued
+            auto flush = [&] {
+                if (r1 > r0 && err[t] == cudaSuccess) {
+                    err[t] = cudaMemcpyAsync(S.Xg.p + r0, S.pin + r0, (r1 - r0) * sizeof(double),
+                                             cudaMemcpyHostToDevice, S.stream);
+                }
+            };
+            each_part(at, slice_begin(total, t, T), slice_begin(total, t + 1, T), [&](size_t m, size_t lo, size_t hi) {
+                if (direct[m]) { return; }
+                if (lo != r1) {
+                    flush();
+                    r0 = lo;
+                }
                 std::memcpy(S.pin + lo, X[m] + (lo - at[m]), (hi - lo) * sizeof(double));
-                err[t] = cudaMemcpyAsync(S.Xg.p + lo, S.pin + lo, (hi - lo) * sizeof(double), cudaMemcpyHostToDevice,
-                                         S.stream);
-            }
+                r1 = hi;
+            });
+            flush();
         });
         for (int t = 0; t < T; ++t) { EGG_CK(err[t]); }
     }
