@@ -1148,17 +1148,25 @@ class Batch : public Session
         return {vec(E), vec(Md)};
     }
 
-    // Per-mesh positions (each flat, global node order of its mesh): views of
-    // one downloaded array, which lives as long as any of them.
+    // Per-mesh positions (each flat, global node order of its mesh), every
+    // array with memory of its own.
     py::list get_X_list()
     {
-        py::array_t<double> all = get_X();
-        double* p = all.mutable_data();
         py::list out;
+        std::vector<double*> ptr;
+        std::vector<int64_t> len;
         for (int m = 0; m < n_; ++m) {
-            out.append(py::array_t<double>({py::ssize_t((offs_[m + 1] - offs_[m]) * dim_)},
-                                           {py::ssize_t(sizeof(double))}, p + offs_[m] * dim_, all));
+            py::array_t<double> x(py::ssize_t((offs_[m + 1] - offs_[m]) * dim_));
+            ptr.push_back(x.mutable_data());
+            len.push_back(int64_t(x.size()));
+            out.append(std::move(x));
         }
+        int rc;
+        {
+            py::gil_scoped_release nogil;
+            rc = egg_b200_batch_get_X(h_.get(), ptr.data(), len.data(), n_);
+        }
+        check(rc);
         return out;
     }
 

@@ -2384,6 +2384,93 @@ static void upload_X(Session& S, const double* const* X, const int64_t* len, int
     S.sync();
 }
 
+// The reverse: every node's position from its owner.  Large page-locked
+// arrays: one DMA each straight into them.  The others: D2H into pinned memory
+// slice by slice, each followed by its event; host thread t waits for slice t
+// only, so the copy-out of early slices overlaps the DMA.
+static void download_X(Session& S, double* const* X, const int64_t* len, int n)
+{
+    const int D = S.dim;
+    EGG_CK(cudaSetDevice(S.device));
+    ensure_xfer(S);
+    if (S.M) {
+        if (D == 2) {
+            scatter_global_kernel<2><<<remap_grid(S.M), 256, 0, S.stream>>>(S.X(S.cur), S.g2s_d.p, S.M, S.Xg.p);
+        } else {
+            scatter_global_kernel<3><<<remap_grid(S.M), 256, 0, S.stream>>>(S.X(S.cur), S.g2s_d.p, S.M, S.Xg.p);
+        }
+        EGG_CK(cudaGetLastError());
+        ++S.launches;
+    }
+    std::vector<size_t> at(size_t(n) + 1, 0);
+    std::vector<char> direct(size_t(n), 0);
+    size_t staged = 0;
+    for (int m = 0; m < n; ++m) {
+        at[size_t(m) + 1] = at[size_t(m)] + size_t(len[m]);
+        direct[size_t(m)] = direct_copy(X[m], len[m], n);
+        if (direct[size_t(m)]) {
+            EGG_CK(cudaMemcpyAsync(X[m], S.Xg.p + at[size_t(m)], size_t(len[m]) * sizeof(double),
+                                   cudaMemcpyDeviceToHost, S.stream));
+        } else {
+            staged += size_t(len[m]);
+        }
+    }
+    if (staged) {
+        ensure_pin(S);
+        const size_t total = at[size_t(n)];
+        const int T = copy_threads(staged * sizeof(double));
+        for (int t = 0; t < T; ++t) {
+            size_t r0 = 0, r1 = 0;
+            auto flush = [&] {
+                if (r1 > r0) {
+                    EGG_CK(cudaMemcpyAsync(S.pin + r0, S.Xg.p + r0, (r1 - r0) * sizeof(double), cudaMemcpyDeviceToHost,
+                                           S.stream));
+                }
+            };
+            each_part(at, slice_begin(total, t, T), slice_begin(total, t + 1, T), [&](size_t m, size_t lo, size_t hi) {
+                if (direct[m]) { return; }
+                if (lo != r1) {
+                    flush();
+                    r0 = lo;
+                }
+                r1 = hi;
+            });
+            flush();
+            EGG_CK(cudaEventRecord(S.xfer_ev[t], S.stream));
+        }
+        cudaError_t err[kMaxCopyThreads] = {};
+        run_slices(T, [&](int t) {
+            err[t] = cudaSetDevice(S.device);
+            if (err[t] == cudaSuccess) { err[t] = cudaEventSynchronize(S.xfer_ev[t]); }
+            if (err[t] != cudaSuccess) { return; }
+            each_part(at, slice_begin(total, t, T), slice_begin(total, t + 1, T), [&](size_t m, size_t lo, size_t hi) {
+                if (!direct[m]) { std::memcpy(X[m] + (lo - at[m]), S.pin + lo, (hi - lo) * sizeof(double)); }
+            });
+        });
+        for (int t = 0; t < T; ++t) { EGG_CK(err[t]); }
+    }
+    S.sync();
+    for (size_t j = 0; j < S.nb_gid.size(); ++j) {
+        const size_t e = size_t(S.nb_gid[j]) * size_t(D);
+        const size_t m = size_t(std::upper_bound(at.begin(), at.end(), e) - at.begin()) - 1;
+        for (int k = 0; k < D; ++k) { X[m][e - at[m] + size_t(k)] = S.nb_val[j * D + k]; }
+    }
+}
+
+// One array per mesh of a batch, each of its mesh's length.
+static void check_mesh_arrays(const Session& S, const double* const* X, const int64_t* len, int32_t n,
+                              const std::string& who)
+{
+    if (S.n_seg <= 0) { invalid(who + ": not a batch session"); }
+    if (n != S.n_seg) { invalid(who + ": one array per mesh is required"); }
+    for (int32_t m = 0; m < n; ++m) {
+        if (len[m] != (S.mesh_node_off[size_t(m) + 1] - S.mesh_node_off[size_t(m)]) * S.dim) {
+            invalid(who + ": mesh " + std::to_string(m) + " has the wrong length");
+        }
+        if (!X[m] && len[m]) { invalid(who + ": NULL array"); }
+    }
+}
+
 // The B-spline seeds after a position reset: NaN (the next projection seeds
 // from its coarse grid), as the reference's upload_X does (src/sweep.hpp:592-597).
 static void reset_seeds(Session& S)
@@ -2811,55 +2898,18 @@ int egg_b200_session_get_X(egg_b200_session* s, double* X, int64_t len)
     return guarded([&] {
         if (!s || !X) { invalid("get_X: NULL argument"); }
         Session& S = *s->impl;
-        const int D = S.dim;
-        if (len != S.M * D) { invalid("get_X: output length " + std::to_string(len) + " != num_nodes*dim"); }
-        EGG_CK(cudaSetDevice(S.device));
-        ensure_xfer(S);
-        const size_t n = size_t(len);
-        if (S.M) {
-            if (D == 2) {
-                scatter_global_kernel<2><<<remap_grid(S.M), 256, 0, S.stream>>>(S.X(S.cur), S.g2s_d.p, S.M, S.Xg.p);
-            } else {
-                scatter_global_kernel<3><<<remap_grid(S.M), 256, 0, S.stream>>>(S.X(S.cur), S.g2s_d.p, S.M, S.Xg.p);
-            }
-            EGG_CK(cudaGetLastError());
-            ++S.launches;
-        }
-        // Page-locked output: one DMA straight into it.
-        cudaPointerAttributes attr {};
-        const bool pinned = cudaPointerGetAttributes(&attr, X) == cudaSuccess && attr.type == cudaMemoryTypeHost;
-        cudaGetLastError();
-        if (pinned && n) {
-            EGG_CK(cudaMemcpyAsync(X, S.Xg.p, n * sizeof(double), cudaMemcpyDeviceToHost, S.stream));
-            EGG_CK(cudaStreamSynchronize(S.stream));
-        }
-        // Otherwise D2H slice by slice, each followed by its event; host thread
-        // t waits for slice t only, so the copy-out of early slices overlaps
-        // the DMA.
-        const int T = pinned ? 0 : copy_threads(n * sizeof(double));
-        if (T) { ensure_pin(S); }
-        for (int t = 0; t < T; ++t) {
-            const size_t a = slice_begin(n, t, T), b = slice_begin(n, t + 1, T);
-            if (b > a) {
-                EGG_CK(cudaMemcpyAsync(S.pin + a, S.Xg.p + a, (b - a) * sizeof(double), cudaMemcpyDeviceToHost,
-                                       S.stream));
-            }
-            EGG_CK(cudaEventRecord(S.xfer_ev[t], S.stream));
-        }
-        cudaError_t err[kMaxCopyThreads] = {};
-        if (T > 0) {
-            run_slices(T, [&](int t) {
-                const size_t a = slice_begin(n, t, T), b = slice_begin(n, t + 1, T);
-                err[t] = cudaSetDevice(S.device);
-                if (err[t] == cudaSuccess) { err[t] = cudaEventSynchronize(S.xfer_ev[t]); }
-                if (err[t] == cudaSuccess && b > a) { std::memcpy(X + a, S.pin + a, (b - a) * sizeof(double)); }
-            });
-        }
-        for (int t = 0; t < T; ++t) { EGG_CK(err[t]); }
-        for (size_t j = 0; j < S.nb_gid.size(); ++j) {
-            for (int k = 0; k < D; ++k) { X[S.nb_gid[j] * D + k] = S.nb_val[j * D + k]; }
-        }
-        S.sync();
+        if (len != S.M * S.dim) { invalid("get_X: output length " + std::to_string(len) + " != num_nodes*dim"); }
+        download_X(S, &X, &len, 1);
+    });
+}
+
+int egg_b200_batch_get_X(egg_b200_session* s, double* const* X, const int64_t* len, int32_t n_meshes)
+{
+    return guarded([&] {
+        if (!s || !X || !len) { invalid("batch_get_X: NULL argument"); }
+        Session& S = *s->impl;
+        check_mesh_arrays(S, X, len, n_meshes, "batch_get_X");
+        download_X(S, X, len, n_meshes);
     });
 }
 
@@ -2878,14 +2928,7 @@ int egg_b200_batch_set_X(egg_b200_session* s, const double* const* X, const int6
     return guarded([&] {
         if (!s || !X || !len) { invalid("batch_set_X: NULL argument"); }
         Session& S = *s->impl;
-        if (S.n_seg <= 0) { invalid("batch_set_X: not a batch session"); }
-        if (n_meshes != S.n_seg) { invalid("batch_set_X: one array per mesh is required"); }
-        for (int32_t m = 0; m < n_meshes; ++m) {
-            if (len[m] != (S.mesh_node_off[size_t(m) + 1] - S.mesh_node_off[size_t(m)]) * S.dim) {
-                invalid("batch_set_X: mesh " + std::to_string(m) + " has the wrong length");
-            }
-            if (!X[m] && len[m]) { invalid("batch_set_X: NULL array"); }
-        }
+        check_mesh_arrays(S, X, len, n_meshes, "batch_set_X");
         upload_X(S, X, len, n_meshes);
     });
 }

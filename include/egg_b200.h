@@ -503,6 +503,9 @@ int egg_b200_session_set_X(egg_b200_session* s, const double* X, int64_t len);
  * m's own node order), without a concatenated copy on the host. */
 int egg_b200_batch_set_X(egg_b200_session* s, const double* const* X, const int64_t* len, int32_t n_meshes);
 
+/* get_X of a batch session into one array per mesh, as batch_set_X takes them. */
+int egg_b200_batch_get_X(egg_b200_session* s, double* const* X, const int64_t* len, int32_t n_meshes);
+
 /* Session facts: [0] dim, [1] global nodes, [2] packed store nodes, [3] moving
  * DOFs, [4] structured-interior DOFs, [5] stored-patch DOFs, [6] owner->copy
  * entries, [7] energy samples, [8] structured energy stencil (0/1),

@@ -39,3 +39,17 @@ def test_positions_come_back(gpu, name, pinned):
         b.set_X(X)
         for x, y in zip(X, b.get_X()):
             np.testing.assert_array_equal(x, y)
+
+
+@pytest.mark.parametrize("name", list(SIDES))
+def test_arrays_own_their_memory(gpu, name):
+    """A mesh that a caller keeps holds nothing of the others."""
+    b = _batch(gpu, SIDES[name])
+    X = b.get_X()
+    for x in X:
+        assert x.flags.owndata and x.base is None and x.flags.writeable
+    keep = X[1].copy()
+    X[0][:] = 7.0
+    np.testing.assert_array_equal(X[1], keep)
+    X[1].resize(2, refcheck=False)
+    np.testing.assert_array_equal(b.get_X()[1], keep)
