@@ -402,7 +402,7 @@ __global__ void __launch_bounds__(TI* TJ* TK, MINB)
 }
 
 // ---------------------------------------------------------------------------
-// Stored-patch sweep, 3D (fp64, general W_inv): one thread per DOF.
+// Stored-patch sweep, 3D (fp64, general W_inv).
 // ---------------------------------------------------------------------------
 struct StoredPatch3 {
     int64_t n;
@@ -524,18 +524,28 @@ __device__ __noinline__ void lattice3_cta(double* P, Lattice3 lat, int64_t d0, c
 }
 
 // Stored-patch sweep, 3D, G lanes per DOF (see stored_patch_kernel): the
-// lanes split the DOF's samples and reduce across the group.  The first `nb`
-// CTAs take the stored DOFs, the others the lattice DOFs.
-template <int KIND, int G, bool CON>
+// lanes split the DOF's samples and reduce across the group.  CLS says what is
+// compiled in: 0 general patches alone, 1 lattice DOFs too, 2 constrained DOFs
+// too.  The first `nb` CTAs take the stored DOFs, the others the lattice DOFs.
+//
+// The lattice part takes a kernel without entity code from 124 to 158
+// registers, 4 to 3 CTAs per SM (with entities it is 236 either way): levels
+// without lattice DOFs, such as every DOF of a target that is no multiple of
+// the identity, launch class 0 (65^3 cube, general target: 700 us a sweep,
+// 775 with one class for both).
+template <int KIND, int G, int CLS>
 __global__ void stored3_kernel(StoredPatch3 sp, int nb, Lattice3 lat, const double* __restrict__ Xin,
                                double* __restrict__ Xout, const double* __restrict__ tau, double delta, double omega,
                                double* __restrict__ grad_out)
 {
-    if (int(blockIdx.x) >= nb) {
-        extern __shared__ __align__(16) unsigned char lat_smem[];
-        lattice3_cta<KIND>(reinterpret_cast<double*>(lat_smem), lat, int64_t(blockIdx.x - nb) * kLatDofs, Xin, Xout,
-                           tau, delta, omega, grad_out);
-        return;
+    constexpr bool CON = CLS == 2;
+    if constexpr (CLS > 0) {
+        if (int(blockIdx.x) >= nb) {
+            extern __shared__ __align__(16) unsigned char lat_smem[];
+            lattice3_cta<KIND>(reinterpret_cast<double*>(lat_smem), lat, int64_t(blockIdx.x - nb) * kLatDofs, Xin,
+                               Xout, tau, delta, omega, grad_out);
+            return;
+        }
     }
     const int lane = threadIdx.x & (G - 1);
     const int64_t ngroups = (int64_t(nb) * blockDim.x) / G;
@@ -605,7 +615,6 @@ __global__ void stored3_kernel(StoredPatch3 sp, int nb, Lattice3 lat, const doub
         // the entity's tangent space, damped by omega before the line
         // search, every trial on the entity; a parametric entity after the
         // first sweep of a run call searches in its parameters.
-        // CON = false (a level without constrained DOFs) compiles none of it.
         const double* er = sp.epar + (etag != 0 ? d * EGG_B200_ENTITY_FIELDS : 0);
         // A B-spline surface carries its foot parameter from sweep to sweep
         // (src/sweep.hpp:1221-1265): the first sweep of a run call steps on

@@ -1611,8 +1611,8 @@ static void launch_stored(Session& S, LevelData& L, const double* xin, double* x
         const int nb = L.n_stored ? int(grid) : 0;
         const unsigned all = unsigned(nb + (L.n_lat + kLatDofs - 1) / kLatDofs);
         const size_t sm = L.n_lat ? size_t(3 * WinLat3::N) * sizeof(double) : 0;
-        auto go3 = [&](auto con) {
-            constexpr bool C = decltype(con)::value;
+        auto go3 = [&](auto cls) {
+            constexpr int C = decltype(cls)::value;
             static_assert(2 * kLatDofs == 128, "one CTA size for both parts");
             switch (G) {
             case 32: stored3_kernel<KIND, 32, C><<<all, 128, sm, st>>>(sp, nb, lat, xin, xout, tau, delta, omega, gout); break;
@@ -1623,9 +1623,11 @@ static void launch_stored(Session& S, LevelData& L, const double* xin, double* x
         };
         S.timed(kKStored, [&] {
             if (L.n_constrained) {
-                go3(std::true_type {});
+                go3(std::integral_constant<int, 2> {});
+            } else if (L.n_lat) {
+                go3(std::integral_constant<int, 1> {});
             } else {
-                go3(std::false_type {});
+                go3(std::integral_constant<int, 0> {});
             }
         });
         return;
