@@ -334,12 +334,12 @@ template <int CI, int CJ> struct TileShared64 {
 };
 
 // Energies of two samples from their squared lengths and dets: s/(2D) each, on
-// one division (shape, untangle with the surrogate dets).
+// one division (untangle with the surrogate dets).
 template <int KIND>
 __device__ __forceinline__ double pair_energy64(double sa, double Da, double sb, double Db, double delta)
 {
     if constexpr (KIND == kShapeSize) {
-        const double ma = sa / (2.0 * Da), mb = sb / (2.0 * Db), da = Da - 1.0, db = Db - 1.0;
+        const double r = 0.5 / (Da * Db), ma = sa * Db * r, mb = sb * Da * r, da = Da - 1.0, db = Db - 1.0;
         return (ma * ma - 1.0 + da * da) + (mb * mb - 1.0 + db * db);
     } else {
         if constexpr (KIND == kUntangle) {
