@@ -407,7 +407,10 @@ __device__ __forceinline__ Support<D> support_of(const CtlTables& T, const CtlNe
 // a few hundred nodes.  WARP: its warp's lanes stride over the box, consecutive
 // lanes along the last axis, and add up by butterfly; otherwise one thread
 // adds in the reference's order, a serial chain of loads (257^2 block, 64^2
-// net: 53 us against 7.5).  Topologies and walled nets keep the serial
+// net: 53 us against 7.5).  With many nets most are done while the last ones
+// iterate; a warp finds which of its controls are left 32 at a time (256 nets,
+// 822 k controls, few of them left: 19 us, 129 one control after another).
+// Topologies and walled nets keep the serial
 // order: their frames amplify a last bit (a sphere's chart near its pole,
 // 7e7-fold), and their nets are small.
 template <int D, bool PRECOND, bool WARP>
@@ -418,9 +421,13 @@ __global__ void ctl_pullback_kernel(CtlTables T, int64_t total_free, const doubl
     constexpr int W = PRECOND ? D * D : D, G = WARP ? 32 : 1;
     const int lane = threadIdx.x & (G - 1);
     const int64_t ngroup = (int64_t(gridDim.x) * blockDim.x) / G;
-    for (int64_t g = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) / G; g < total_free; g += ngroup) {
-        const int ni = net_of(T.free_pfx, T.n_nets, g);
-        if (st && !PRECOND && st[ni].done) { continue; }
+    const int64_t g0 = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) / G;
+    auto active = [&](int64_t g, int& ni) {
+        if (g >= total_free) { return false; }
+        ni = net_of(T.free_pfx, T.n_nets, g);
+        return PRECOND || st == nullptr || !st[ni].done;
+    };
+    auto pull = [&](int64_t g, int ni) {
         const CtlNet n = T.nets[ni];
         int a[3] = {0, 0, 0};
 #pragma unroll
@@ -456,6 +463,22 @@ __global__ void ctl_pullback_kernel(CtlTables T, int64_t total_free, const doubl
         if (lane == 0) {
 #pragma unroll
             for (int i = 0; i < W; ++i) { out[g * W + i] = acc[i]; }
+        }
+    };
+    int ni = 0;
+    if constexpr (WARP) {
+        // a warp's controls of 32 rounds at once: each lane looks one of them up
+        for (int64_t b = g0; b < total_free; b += 32 * ngroup) {
+            unsigned todo = __ballot_sync(0xffffffffu, active(b + lane * ngroup, ni));
+            while (todo != 0u) {
+                const int q = __ffs(int(todo)) - 1;
+                todo &= todo - 1u;
+                pull(b + q * ngroup, __shfl_sync(0xffffffffu, ni, q));
+            }
+        }
+    } else {
+        for (int64_t g = g0; g < total_free; g += ngroup) {
+            if (active(g, ni)) { pull(g, ni); }
         }
     }
 }
