@@ -196,8 +196,7 @@ struct Session : LevelData {
     int dim = 2;
     int prec = EGG_B200_PREC_FP64;
     int device = 0;
-    int num_sms = 148;
-        cudaStream_t stream = nullptr;
+    cudaStream_t stream = nullptr;
     // side stream + fork/join events: the stored-patch sweep runs beside the
     // interior tiles (both read the frozen snapshot, write disjoint slots)
     cudaStream_t side = nullptr;
@@ -1283,7 +1282,6 @@ static Session* create_session(const egg_b200_session_desc& d)
     EGG_CK(cudaEventCreateWithFlags(&S->fork_ev, cudaEventDisableTiming));
     EGG_CK(cudaEventCreateWithFlags(&S->join_ev, cudaEventDisableTiming));
     configure_kernels(S->prec, S->dim);
-    EGG_CK(cudaDeviceGetAttribute(&S->num_sms, cudaDevAttrMultiProcessorCount, S->device));
 
     // ---- upload -----------------------------------------------------------
     S->es_W.upload(es_W_h);
