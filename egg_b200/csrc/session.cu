@@ -1697,6 +1697,11 @@ template <int KIND> static void launch_reduce(Session& S, const double* x, doubl
     double* pc = ps + S.red_grid;
     double* pm = pc + S.red_grid;
     const ReduceOut out {out_e, out_m, S.red_ticket.p};
+    // no more CTAs than one item a thread takes: every CTA's ticket is an atomic
+    // on one word, and a small store's energy() waited 4 us for those of idle
+    // CTAs (65^2: 39.8 us a call, 33.8 now); their empty partials add nothing
+    const int64_t items = S.es_struct ? S.es_ncell : S.es_ns;
+    const int grid = int(std::min<int64_t>(S.red_grid, std::max<int64_t>(1, (items + 255) / 256)));
     const auto* X2 = reinterpret_cast<const double2*>(x);
     if (S.es_struct) {
         EnergyStructured2 es;
@@ -1710,18 +1715,18 @@ template <int KIND> static void launch_reduce(Session& S, const double* x, doubl
         es.wt_stride = S.es_wtstride;
         if (S.dim == 3) {
             S.timed(kKReduce, [&] {
-                energy_structured3_kernel<KIND><<<S.red_grid, 256, 0, S.stream>>>(es, x, delta, ps, pc, pm, out);
+                energy_structured3_kernel<KIND><<<grid, 256, 0, S.stream>>>(es, x, delta, ps, pc, pm, out);
             });
         } else {
             S.timed(kKReduce, [&] {
-                energy_structured2_kernel<KIND><<<S.red_grid, 256, 0, S.stream>>>(es, X2, delta, ps, pc, pm, out);
+                energy_structured2_kernel<KIND><<<grid, 256, 0, S.stream>>>(es, X2, delta, ps, pc, pm, out);
             });
         }
     } else if (S.dim == 3) {
         EnergyStored3 es {S.es_ns,  S.es_gc.p, S.es_gn0.p,    S.es_gn1.p, S.es_gn2.p,     S.es_s0.p,
                           S.es_s1.p, S.es_s2.p, S.es_W.p, S.es_wstride, S.es_wt.p, S.es_wtstride};
         S.timed(kKReduce, [&] {
-            energy_stored3_kernel<KIND><<<S.red_grid, 256, 0, S.stream>>>(es, x, delta, ps, pc, pm, out);
+            energy_stored3_kernel<KIND><<<grid, 256, 0, S.stream>>>(es, x, delta, ps, pc, pm, out);
         });
     } else {
         EnergyStored2 es;
@@ -1736,7 +1741,7 @@ template <int KIND> static void launch_reduce(Session& S, const double* x, doubl
         es.wt = S.es_wt.p;
         es.wt_stride = S.es_wtstride;
         S.timed(kKReduce, [&] {
-            energy_stored2_kernel<KIND><<<S.red_grid, 256, 0, S.stream>>>(es, X2, delta, ps, pc, pm, out);
+            energy_stored2_kernel<KIND><<<grid, 256, 0, S.stream>>>(es, X2, delta, ps, pc, pm, out);
         });
     }
     launch_soft_energy(S, x, out_e);
