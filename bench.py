@@ -44,7 +44,7 @@ BYTES_PER_UPDATE = 2 * 2 * 8
 # of a 2049^2 launch (4,190,209 DOFs; the store exceeds L2): traffic and
 # instructions grow in proportion to the DOFs swept.
 DRAM_BYTES_PER_UPDATE = 527.0e6 / 16769025
-INSTR_PER_UPDATE = 1000.0
+INSTR_PER_UPDATE = 1014.0
 # Issue roof: 148 SMs x 4 schedulers x 32 lanes, one warp instruction per
 # scheduler per cycle.
 ISSUE_LANES = 148 * 4 * 32

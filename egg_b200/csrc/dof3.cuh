@@ -33,7 +33,8 @@
 // d_jk^2, kb = (n_i + n_j) t_k - ..., (n_i + n_j) I - ...) the same quantities
 // cancel to (short / long)^2 of their terms where a cell's edges differ in
 // length or lie near one line: the fp32 step of 1 : 0.01 : 0.01 cells was then
-// off by 9e-4 of the short spacing (median), and is by 8e-7 in this form.
+// off by 8e-4 of the short spacing (median), and is by 8e-7 in this form, for
+// 3% of the kernel (129^3 cube, mixed: 545 us a sweep, now 560).
 //
 // V is double, or F2: two fp32 lanes evaluated by one instruction (x2.cuh).
 // The lanes are the two sides of an axis group, and the two directions of

@@ -116,9 +116,9 @@ constexpr int kMaxCopyThreads = 16;
 constexpr Variant kVar64[kNumVariants] = {{8, 16, 1, 4, 1}, {8, 16, 1, 4, 4}, {8, 16, 1, 5, 1}, {16, 16, 1, 2, 1}, {8, 16, 1, 3, 1}};
 constexpr Variant kVar32[kNumVariants] = {{8, 16, 1, 7, 2}, {8, 16, 1, 8, 2}, {8, 16, 1, 6, 2}, {8, 16, 1, 5, 2}, {4, 24, 1, 9, 2}};
 // 3D (interior3_kernel), us a sweep of a 129^3 / 59^3 / 33^3 cube, in the table's
-// order: fp64 969 / 125 / 25.0, 957 / 112 / 26.9, 963 / 120 / 27.0,
-// 1029 / 120 / 28.3, 975 / 125 / 27.2; mixed 545 / 72 / 16.8, 556 / 72 / 16.7,
-// 559 / 74 / 16.7, 558 / 69 / 17.1, 582 / 73 / 17.0.
+// order: fp64 991 / 127 / 26.9, 976 / 116 / 26.9, 1004 / 125 / 28.2,
+// 1070 / 125 / 29.2, 971 / 124 / 26.9; mixed 560 / 70 / 16.7, 571 / 68 / 18.1,
+// 575 / 74 / 16.7, 573 / 68 / 18.7, 588 / 73 / 16.7.
 constexpr Variant kVar3_64[kNumVariants] = {{4, 8, 8, 2}, {2, 4, 16, 4}, {4, 4, 8, 4}, {2, 4, 8, 8}, {2, 8, 16, 2}};
 constexpr Variant kVar3_32[kNumVariants] = {{4, 4, 8, 4}, {2, 4, 16, 4}, {4, 8, 8, 2}, {4, 4, 4, 8}, {2, 8, 16, 2}};
 

@@ -529,17 +529,17 @@ int egg_b200_session_reset_stats(egg_b200_session* s);
 int egg_b200_session_checkpoint(egg_b200_session* s);
 int egg_b200_session_restore(egg_b200_session* s);
 
-/* Autotuner of the interior sweep kernel: times each launch variant (cells
+/* Autotuner of the interior sweep kernel: times each launch variant (DOFs
  * per CTA, resident CTAs per SM) on the session's own resident data without
  * changing it, keeps the fastest and returns its index.  Runs automatically
  * before the first sweep unless EGG_B200_AUTOTUNE=0.  No counterpart in the
  * reference (AdaptiveCpp picks launch shapes itself). */
 int egg_b200_session_autotune(egg_b200_session* s, int32_t objective, int32_t reps, int32_t* chosen);
 int egg_b200_session_set_variant(egg_b200_session* s, int32_t variant);
-/* Current variant, per-variant shape (ci, cj, ck, min CTAs/SM, full_dof)
- * [5*n] -- 2D: cells per CTA, or DOFs per CTA when full_dof = 1; 3D: DOFs per
- * CTA -- and the tuned times in ms [n], for the first n <=
- * EGG_B200_NUM_VARIANTS variants. */
+/* Current variant, per-variant shape (ci, cj, ck, min CTAs/SM, form) [5*n] --
+ * ci x cj (x ck) DOFs per CTA; form, 2D only: 1 fp64 with a thread per DOF, 4
+ * fp64 with a thread per cell, 2 packed fp32 pairs; 0 in 3D -- and the tuned
+ * times in ms [n], for the first n <= EGG_B200_NUM_VARIANTS variants. */
 #define EGG_B200_NUM_VARIANTS 5
 int egg_b200_session_variant_info(egg_b200_session* s, int32_t* variant, int32_t* shape, double* times_ms,
                                   int32_t n);
